@@ -199,6 +199,14 @@ int vtb_compute_G(const double* tk1, const double* tk2, const int32_t* ind, int 
                   const double* Dsw, int64_t dsw_ld, double lamb, int lower_only, double* G, int64_t G_ld,
                   void* stream);
 
+/* vtb_compute_G with a workspace for the intervals' harmonics (8 n (2Mt+1)
+ * bytes, vtb_compute_G_workspace), which are then formed once per interval
+ * instead of once per output tile. */
+int vtb_compute_G_workspace(int n, int Mt, int64_t* bytes);
+int vtb_compute_G_work(const double* tk1, const double* tk2, const int32_t* ind, int n, double Wt, int Mt,
+                       const double* Dsw, int64_t dsw_ld, double lamb, int lower_only, double* G, int64_t G_ld,
+                       void* work, int64_t work_bytes, void* stream);
+
 /* Workspace bytes of vtb_solve_eq_sym for order n. */
 int vtb_solve_eq_sym_workspace(int n, int64_t* bytes);
 

@@ -44,6 +44,8 @@ SIGNATURES = {
     "vtb_dsw": [P, I, I, P, P, L, P],
     "vtb_compute_q": [P, P, P, I, P, P, P, P, P, P],
     "vtb_compute_G": [P, P, P, I, D, I, P, L, D, I, P, L, P],
+    "vtb_compute_G_workspace": [I, I, P],
+    "vtb_compute_G_work": [P, P, P, I, D, I, P, L, D, I, P, L, P, L, P],
     "vtb_solve_eq_sym_workspace": [I, P],
     "vtb_solve_eq_sym": [P, L, P, P, I, D, P, L, P, P],
     "vtb_rnn": [P, L, P, P, P, P, I, D, I, P, I, P],

@@ -15,7 +15,7 @@
 //      vrf.py:502-559), as one real GEMM over the interleaved (re, im) planes.
 //  vtb_compute_q : compute_q_Kernel (vtem/dirichlet.py:204-222).
 //  vtb_compute_G : compute_G_Kernel + diag_add_Kernel (dirichlet.py:272-350),
-//      same per-element formula, 2-D tiled.
+//      the same entries as products of the intervals' harmonics.
 #include "common.cuh"
 #include "gemm_f64.cuh"
 
@@ -163,49 +163,235 @@ __global__ void compute_q_kernel(const double* __restrict__ tk1, const double* _
     }
 }
 
-__device__ __forceinline__ double g_time(double tk1, double tk2, double tl1, double tl2, int M, double WM) {
-    double sum = 0;
-    for (int m = 1; m <= M; ++m) {
-        sum += (cos(m * WM * (tk2 - tl2)) - cos(m * WM * (tk2 - tl1)) - cos(m * WM * (tk1 - tl2)) +
-                cos(m * WM * (tk1 - tl1))) /
-               (m * m);
+// G[r][c] = Dsw[ind_r][ind_c] int_r int_c D(s - t) ds dt with the Dirichlet
+// kernel D.  compute_G_Kernel's bracket (dirichlet.py:300-320)
+//   sum_m [cos mW(r2-c2) - cos mW(r2-c1) - cos mW(r1-c2) + cos mW(r1-c1)] 2/(mW)^2 + |r||c|
+// is the product of two (2Mt+1)-vectors, one per interval:
+//   |r||c| + 2 sum_m Re T_r(m) conj T_c(m),
+//   T_k(m) = int_{tk1}^{tk2} e^{jmWs} ds = (2/(mW)) sin(mW d/2) e^{jmW tbar},
+// so an entry costs 2Mt+1 float64 FMAs instead of 4 Mt cosines, and no
+// difference of cosines cancels.  Only differences of times count: they are
+// taken from the first interval's start, so that an offset common to all
+// costs no phase.  Bound: the HBM write of G (n^2 * 8 bytes).
+//
+// A block forms 64 x 64 tiles of the lower triangle of tiles on the float64
+// tensor-core path (mma m8n8k4, exact float64 FMAs: few shared-memory reads
+// and instructions per entry, which a register tile with bounds checks and
+// gathers per entry was bound by), stages the products in shared memory and
+// writes them by whole rows (256 bytes a warp), times Dsw, and, unless only
+// the lower triangle is wanted, again transposed as the mirror tile: half the
+// products.  A block walks `strip` tiles of one tile row and keeps that row's
+// harmonics.
+//
+// The harmonics (two sincos, a division and two complex products per
+// harmonic, a fresh sincos every kGHarm so that powers lose a few ulp at any
+// Mt) are formed once per interval in the caller's workspace
+// (harmonics_table_kernel), or, without one, by every tile that meets the
+// interval.  Measured at n = 24001, Mt = 8 (4.6 GB): 41.6 ms with the cosines,
+// 1.51 ms with a register tile on the FMA pipe, 1.31 ms here (3.5 TB/s; with
+// rows of whole sectors, n = 24000, 1.06 ms, where a fill takes 0.62): the odd
+// row length's split sectors and the latency of a tile's phases, four blocks
+// per SM.  Three blocks with deeper gathers: 1.36 ms; strips of 16: 1.36 ms.
+constexpr int kGT = 64;        // tile side
+constexpr int kGHarm = 8;      // harmonics per pass over the tile
+constexpr int kGF = 2 * kGHarm + 1;
+constexpr int kGK = 20;        // kGF up to whole k-steps of 4
+constexpr int kGS = kGT + 4;   // row stride of the staged harmonics: fragment reads free of bank conflicts
+
+// place of entry (r, c) of the staged products: rows, columns and the
+// products' 4 x 4 fragment corners all free of bank conflicts
+__device__ __forceinline__ int g_at(int r, int c) { return r * kGT + (c ^ (((r & 3) << 2) | ((r >> 2) & 3))); }
+
+// place of tile column c among the staged harmonics: a product's 8 columns
+// 2q, 2q + 1 hold the tile's q, q + 4, so that a fragment's stores are contiguous
+__device__ __forceinline__ int g_col(int c) { return (c & ~7) | ((c & 3) << 1) | ((c >> 2) & 1); }
+
+// Harmonics m0 .. m0+kGHarm-1 (m >= 1; zero beyond Mt) of the interval (a, b),
+// scaled: f[S * (2i + 1)] = Re, f[S * (2i + 2)] = Im, and f[0] = b - a in the first pass.
+template <int S>
+__device__ __forceinline__ void g_features(double a, double b, int m0, int Mt, double W, double scale,
+                                           double* __restrict__ f) {
+    const double d = b - a, tb = 0.5 * (a + b);
+    f[0] = m0 == 1 ? d : 0.0;
+    double s1, c1, sh, ch, sp, cp, sq, cq;
+    sincos(W * tb, &s1, &c1);
+    sincos(0.5 * W * d, &sh, &ch);
+    if (m0 == 1) {
+        sp = s1;
+        cp = c1;
+        sq = sh;
+        cq = ch;
+    } else {
+        sincos(m0 * W * tb, &sp, &cp);
+        sincos(m0 * (0.5 * W) * d, &sq, &cq);
     }
-    sum = sum * 2 / (WM * WM) + (tk2 - tk1) * (tl2 - tl1);
-    return sum;
+#pragma unroll
+    for (int i = 0; i < kGHarm; ++i) {
+        const int m = m0 + i;
+        const double amp = m <= Mt ? scale * (2.0 / (m * W)) * sq : 0.0;
+        f[S * (2 * i + 1)] = amp * cp;
+        f[S * (2 * i + 2)] = amp * sp;
+        const double c2 = cp * c1 - sp * s1, s2 = cp * s1 + sp * c1;
+        const double c3 = cq * ch - sq * sh, s3 = cq * sh + sq * ch;
+        cp = c2;
+        sp = s2;
+        cq = c3;
+        sq = s3;
+    }
 }
 
-// 32x32 output tile per block of 256 threads (each thread 4 rows of one column).
-__global__ void __launch_bounds__(256) compute_G_kernel(const double* __restrict__ tk1, const double* __restrict__ tk2,
-                                                        const int32_t* __restrict__ ind, int n, double WM, int Mt,
-                                                        const double* __restrict__ Dsw, int64_t dsw_ld, double lamb,
-                                                        int lower_only, double* __restrict__ G, int64_t G_ld) {
-    __shared__ double r1[32], r2[32], c1[32], c2[32];
-    __shared__ int ri[32], ci[32];
-    const int row0 = blockIdx.y * 32, col0 = blockIdx.x * 32;
-    if (lower_only && col0 > row0 + 31) return;
-    const int tid = threadIdx.x;
-    if (tid < 32) {
-        const int r = row0 + tid;
-        r1[tid] = r < n ? tk1[r] : 0.0;
-        r2[tid] = r < n ? tk2[r] : 0.0;
-        ri[tid] = r < n ? ind[r] : 0;
-    } else if (tid < 64) {
-        const int c = col0 + tid - 32;
-        c1[tid - 32] = c < n ? tk1[c] : 0.0;
-        c2[tid - 32] = c < n ? tk2[c] : 0.0;
-        ci[tid - 32] = c < n ? ind[c] : 0;
+// table[(k) * n + i]: feature k = 0..2Mt of interval i, unscaled
+__global__ void __launch_bounds__(128) harmonics_table_kernel(const double* __restrict__ tk1,
+                                                              const double* __restrict__ tk2, int n, double W, int Mt,
+                                                              double* __restrict__ table) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m0 = 1 + blockIdx.y * kGHarm;
+    if (i >= n) return;
+    const double t0 = tk1[0];
+    double f[kGF];
+    g_features<1>(tk1[i] - t0, tk2[i] - t0, m0, Mt, W, 1.0, f);
+    if (m0 == 1) table[i] = f[0];
+#pragma unroll
+    for (int h = 0; h < kGHarm; ++h) {
+        const int m = m0 + h;
+        if (m <= Mt) {
+            table[(int64_t)(2 * m - 1) * n + i] = f[2 * h + 1];
+            table[(int64_t)(2 * m) * n + i] = f[2 * h + 2];
+        }
     }
-    __syncthreads();
-    const int lc = tid % 32;
-    const int col = col0 + lc;
-    if (col >= n) return;
-    for (int rr = tid / 32; rr < 32; rr += 8) {
-        const int row = row0 + rr;
-        if (row >= n) break;
-        if (lower_only && col > row) continue;
-        double v = g_time(r1[rr], r2[rr], c1[lc], c2[lc], Mt, WM) * Dsw[(int64_t)ri[rr] * dsw_ld + ci[lc]];
-        if (row == col && lamb != 0.0) v += lamb;
-        G[(int64_t)row * G_ld + col] = v;
+}
+
+// features of the tile's intervals i0 .. i0+kGT-1 for the pass from harmonic m0, from the table (zero-padded to kGK)
+template <bool COLS>
+__device__ __forceinline__ void g_load(const double* __restrict__ table, int n, int i0, int m0, int nf, double scale,
+                                       double* __restrict__ f) {
+    for (int e = threadIdx.x; e < kGK * kGT; e += 256) {
+        const int k = e / kGT, i = e % kGT;
+        double v = 0.0;
+        if (i0 + i < n && k < nf && (k > 0 || m0 == 1)) {
+            v = __ldg(table + (int64_t)(k + (k > 0 ? 2 * (m0 - 1) : 0)) * n + i0 + i);
+            if (k > 0) v *= scale;
+        }
+        f[k * kGS + (COLS ? g_col(i) : i)] = v;
+    }
+}
+
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Rows w, w + 8, ... of a staged tile times Dsw into G, one row of 64 entries
+// at a time by a warp.  TRANS: the mirror tile (tile columns become G's rows).
+// EDGE: the tile crosses G's edge or its diagonal.
+template <bool TRANS, bool EDGE>
+__device__ __forceinline__ void g_store(const double* __restrict__ tile, const int* __restrict__ ri,
+                                        const int* __restrict__ ci, int r0, int c0, int n,
+                                        const double* __restrict__ Dsw, int64_t dsw_ld, double lamb, int lower_only,
+                                        double* __restrict__ G, int64_t G_ld) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k0 = ci[lane], k1 = ci[lane + 32];
+#pragma unroll 4
+    for (int r = w; r < kGT; r += 8) {
+        const double v0 = tile[TRANS ? g_at(lane, r) : g_at(r, lane)];
+        const double v1 = tile[TRANS ? g_at(lane + 32, r) : g_at(r, lane + 32)];
+        const double* dr = Dsw + (int64_t)ri[r] * dsw_ld;
+        double* g = G + (int64_t)(r0 + r) * G_ld + c0 + lane;
+        if (!EDGE) {
+            __stcs(g, v0 * __ldg(dr + k0));
+            __stcs(g + 32, v1 * __ldg(dr + k1));
+        } else if (r0 + r < n) {
+            const int row = r0 + r, a = c0 + lane, b = a + 32;
+            if (a < n && !(lower_only && a > row)) __stcs(g, v0 * __ldg(dr + k0) + (a == row ? lamb : 0.0));
+            if (b < n && !(lower_only && b > row)) __stcs(g + 32, v1 * __ldg(dr + k1) + (b == row ? lamb : 0.0));
+        }
+    }
+}
+
+template <bool TABLE>
+__global__ void __launch_bounds__(256, 4) compute_G_kernel(const double* __restrict__ tk1, const double* __restrict__ tk2,
+                                                           const int32_t* __restrict__ ind, int n, double W, int Mt,
+                                                           const double* __restrict__ Dsw, int64_t dsw_ld, double lamb,
+                                                           int lower_only, int strip,
+                                                           const double* __restrict__ table, double* __restrict__ G,
+                                                           int64_t G_ld) {
+    extern __shared__ double gsm[];
+    double* fr = gsm;                       // kGK x kGS: the tile row's harmonics
+    double* fc = fr + kGK * kGS;            // kGK x kGS: the tile column's, doubled
+    double* tile = fc + kGK * kGS;          // kGT x kGT: the products
+    __shared__ int ri[kGT], ci[kGT];
+    // block -> (tile row, strip of tile columns): tile rows in groups of `strip`
+    // rows, group g having g + 1 strips a row
+    int g = (int)((sqrt(1.0 + 8.0 * (double)blockIdx.x / strip) - 1.0) * 0.5);
+    while ((int64_t)strip * g * (g + 1) / 2 > blockIdx.x) --g;
+    while ((int64_t)strip * (g + 1) * (g + 2) / 2 <= blockIdx.x) ++g;
+    const int rem = (int)(blockIdx.x - (int64_t)strip * g * (g + 1) / 2);
+    const int ti = g * strip + rem / (g + 1);
+    const int tj0 = (rem % (g + 1)) * strip;
+    const int row0 = ti * kGT;
+    if (row0 >= n) return;
+    const int tid = threadIdx.x;
+    const double t0 = TABLE ? 0.0 : tk1[0];
+    // warp (wr, wc) of 2 x 4: 32 rows x 16 columns as 4 x 2 products of 8 x 8
+    const int lane = tid & 31, wr = (tid >> 5) & 1, wc = tid >> 6;
+    const int fl = (lane & 3) * kGS + (lane >> 2);
+    if (tid < kGT) ri[tid] = row0 + tid < n ? ind[row0 + tid] : 0;
+    if (!TABLE)
+        for (int e = tid; e < (kGK - kGF) * kGS; e += 256) fr[kGF * kGS + e] = fc[kGF * kGS + e] = 0.0;
+    for (int tj = tj0; tj < min(tj0 + strip, ti + 1); ++tj) {
+        const int col0 = tj * kGT;
+        double acc[4][2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int m0 = 1; m0 <= Mt; m0 += kGHarm) {
+            __syncthreads();                // the previous pass's harmonics and the previous tile have been read
+            const int nf = 1 + 2 * min(kGHarm, Mt + 1 - m0);
+            const bool rows = tj == tj0 || Mt > kGHarm;
+            if (TABLE) {
+                g_load<true>(table, n, col0, m0, nf, 2.0, fc);
+                if (rows) g_load<false>(table, n, row0, m0, nf, 1.0, fr);
+            } else if (tid < kGT) {
+                const int c = col0 + tid;
+                g_features<kGS>(c < n ? tk1[c] - t0 : 0.0, c < n ? tk2[c] - t0 : 0.0, m0, Mt, W, 2.0,
+                                fc + g_col(tid));
+            } else if (tid < 2 * kGT && rows) {
+                const int r = row0 + tid - kGT;
+                g_features<kGS>(r < n ? tk1[r] - t0 : 0.0, r < n ? tk2[r] - t0 : 0.0, m0, Mt, W, 1.0, fr + tid - kGT);
+            }
+            if (m0 == 1 && tid >= 192) ci[tid - 192] = col0 + tid - 192 < n ? ind[col0 + tid - 192] : 0;
+            __syncthreads();
+            const double* fa = fr + fl + 32 * wr;
+            const double* fb = fc + fl + 16 * wc;
+            for (int k = 0; k < nf; k += 4, fa += 4 * kGS, fb += 4 * kGS) {
+                const double b0 = fb[0], b1 = fb[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double a = fa[8 * i];
+                    dmma_8x8x4(acc[i][0], a, b0);
+                    dmma_8x8x4(acc[i][1], a, b1);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int r = 32 * wr + 8 * i + (lane >> 2), c = 16 * wc + 8 * j + (lane & 3);
+                tile[g_at(r, c)] = acc[i][j][0];
+                tile[g_at(r, c + 4)] = acc[i][j][1];
+            }
+        __syncthreads();
+        if (ti == tj || row0 + kGT > n || col0 + kGT > n) {
+            g_store<false, true>(tile, ri, ci, row0, col0, n, Dsw, dsw_ld, lamb, lower_only, G, G_ld);
+            if (!lower_only && ti != tj)
+                g_store<true, true>(tile, ci, ri, col0, row0, n, Dsw, dsw_ld, lamb, 0, G, G_ld);
+        } else {
+            g_store<false, false>(tile, ri, ci, row0, col0, n, Dsw, dsw_ld, lamb, 0, G, G_ld);
+            if (!lower_only) g_store<true, false>(tile, ci, ri, col0, row0, n, Dsw, dsw_ld, lamb, 0, G, G_ld);
+        }
     }
 }
 
@@ -271,15 +457,53 @@ VTB_API int vtb_compute_q(const double* tk1, const double* tk2, const int32_t* i
     return launch_status();
 }
 
+static int launch_G(const double* tk1, const double* tk2, const int32_t* ind, int n, double Wt, int Mt,
+                    const double* Dsw, int64_t dsw_ld, double lamb, int lower_only, double* table, double* G,
+                    int64_t G_ld, cudaStream_t s) {
+    const int T = ceil_div(n, kGT);
+    VTB_CHECK_ARG(ceil_div(n, 32) <= 65535);
+    // one tile a block while that is at most two waves of four blocks per SM,
+    // else four (the row's harmonics formed or read once for four tiles)
+    const int strip = (int64_t)T * (T + 1) / 2 <= 8 * kNumSMs ? 1 : 4;
+    const int64_t groups = ceil_div(T, strip);
+    const unsigned blocks = (unsigned)(strip * groups * (groups + 1) / 2);
+    const size_t sm = (size_t)(2 * kGK * kGS + kGT * kGT) * sizeof(double);
+    const double W = Wt / Mt;
+    if (table) {
+        harmonics_table_kernel<<<dim3(ceil_div(n, 128), ceil_div(Mt, kGHarm)), 128, 0, s>>>(tk1, tk2, n, W, Mt, table);
+        VTB_CUDA_TRY(cudaFuncSetAttribute(compute_G_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        compute_G_kernel<true><<<blocks, 256, sm, s>>>(tk1, tk2, ind, n, W, Mt, Dsw, dsw_ld, lamb, lower_only, strip,
+                                                       table, G, G_ld);
+    } else {
+        VTB_CUDA_TRY(cudaFuncSetAttribute(compute_G_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        compute_G_kernel<false><<<blocks, 256, sm, s>>>(tk1, tk2, ind, n, W, Mt, Dsw, dsw_ld, lamb, lower_only, strip,
+                                                        nullptr, G, G_ld);
+    }
+    return launch_status();
+}
+
 VTB_API int vtb_compute_G(const double* tk1, const double* tk2, const int32_t* ind, int n, double Wt, int Mt,
                           const double* Dsw, int64_t dsw_ld, double lamb, int lower_only, double* G, int64_t G_ld,
                           void* stream) {
     VTB_CHECK_ARG(n >= 0 && Mt >= 0 && G_ld >= n);
     if (n == 0) return VTB_OK;
     VTB_CHECK_ARG(tk1 && tk2 && ind && Dsw && G && Mt > 0);
-    dim3 grid(ceil_div(n, 32), ceil_div(n, 32));
-    VTB_CHECK_ARG(grid.y <= 65535);
-    compute_G_kernel<<<grid, 256, 0, as_stream(stream)>>>(tk1, tk2, ind, n, Wt / Mt, Mt, Dsw, dsw_ld, lamb,
-                                                         lower_only, G, G_ld);
-    return launch_status();
+    return launch_G(tk1, tk2, ind, n, Wt, Mt, Dsw, dsw_ld, lamb, lower_only, nullptr, G, G_ld, as_stream(stream));
+}
+
+VTB_API int vtb_compute_G_workspace(int n, int Mt, int64_t* bytes) {
+    VTB_CHECK_ARG(n >= 0 && Mt > 0 && bytes);
+    *bytes = (int64_t)n * (2 * (int64_t)Mt + 1) * 8;
+    return VTB_OK;
+}
+
+VTB_API int vtb_compute_G_work(const double* tk1, const double* tk2, const int32_t* ind, int n, double Wt, int Mt,
+                               const double* Dsw, int64_t dsw_ld, double lamb, int lower_only, double* G, int64_t G_ld,
+                               void* work, int64_t work_bytes, void* stream) {
+    VTB_CHECK_ARG(n >= 0 && Mt >= 0 && G_ld >= n);
+    if (n == 0) return VTB_OK;
+    VTB_CHECK_ARG(tk1 && tk2 && ind && Dsw && G && Mt > 0 && work && ((uintptr_t)work & 7) == 0);
+    VTB_CHECK_ARG(work_bytes >= (int64_t)n * (2 * (int64_t)Mt + 1) * 8 && ceil_div(Mt, kGHarm) <= 65535);
+    return launch_G(tk1, tk2, ind, n, Wt, Mt, Dsw, dsw_ld, lamb, lower_only, reinterpret_cast<double*>(work), G, G_ld,
+                    as_stream(stream));
 }

@@ -73,9 +73,10 @@ class dirichlet(object):
         all the pseudoinverse solve reads."""
         Dsw = _dev(_load(Dswfilename))
         self.d_G = torch.empty((self.size, self.size), dtype=F64, device="cuda")
-        call("vtb_compute_G", dptr(self.d_tk1), dptr(self.d_tk2), dptr(self.d_neuron_ind), self.size, self.Wt,
+        work = torch.empty(8 * self.size * (2 * max(self.Mt, 0) + 1), dtype=torch.uint8, device="cuda")
+        call("vtb_compute_G_work", dptr(self.d_tk1), dptr(self.d_tk2), dptr(self.d_neuron_ind), self.size, self.Wt,
              self.Mt, dptr(Dsw), Dsw.shape[1], float(lamb), int(bool(lower_only)), dptr(self.d_G), self.size,
-             stream_ptr())
+             dptr(work), work.numel(), stream_ptr())
 
     def compute_Gb(self, Dsfilename, lamb=0.0, lower_only=False):
         """Gram from the Dirichlet coefficients (dirichlet.py:87-126): the
