@@ -235,6 +235,14 @@ int vtb_reconstruct(const double* dirich, int N, int P, const double* tk1, const
                     const double* c, const int32_t* ind, const double* norm, int nspk, const double* t, int Nt,
                     int Mt, double WM, double* u, void* work, int64_t work_bytes, void* stream);
 
+/* vtb_reconstruct at the uniform times t0 + f dt, f = 0..Nt-1, Mt in 1..10:
+ * the neurons are summed once into 2Mt+1 spatial weights per pixel, and each
+ * voxel is their product with the harmonics at its time. */
+int vtb_reconstruct_uniform_workspace(int N, int P, int Mt, int64_t* bytes);
+int vtb_reconstruct_uniform(const double* dirich, int N, int P, const double* tk1, const double* tk2, const double* c,
+                            const int32_t* ind, const double* norm, int nspk, double t0, double dt, int Nt, int Mt,
+                            double WM, double* u, void* work, int64_t work_bytes, void* stream);
+
 /* ------------------------------------------------------------ coefficient-space decoder
  *
  * The same reconstruction as compute_q + compute_G + solve_eq_sym +

@@ -121,7 +121,6 @@ class dirichlet(object):
         held in ``self.d_q``, at t = arange(time_frame[0], time_frame[1], dt)
         (dirichlet.py:165-189)."""
         t = np.arange(time_frame[0], time_frame[1], dt)
-        d_t = _dev(t)
         dirich = _dev(_load(dirichfilename))
         N, Py, Px = dirich.shape
         c = self.d_q.reshape(-1).contiguous()
@@ -129,10 +128,17 @@ class dirichlet(object):
         if perm is not None:
             c = c[perm].contiguous()
         nbytes = np.zeros(1, np.int64)
-        from . import _abi
-        _abi.lib().vtb_reconstruct_workspace(N, len(t), self.Mt, nbytes.ctypes.data)
-        work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device="cuda")
         u = torch.empty((len(t), Py, Px), dtype=F64, device="cuda")
+        if 1 <= self.Mt <= 10:
+            call("vtb_reconstruct_uniform_workspace", N, Py * Px, self.Mt, nbytes.ctypes.data)
+            work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device="cuda")
+            call("vtb_reconstruct_uniform", dptr(dirich), N, Py * Px, dptr(tk1), dptr(tk2), dptr(c), dptr(ind),
+                 dptr(self.d_norm), self.size, float(time_frame[0]), float(dt), len(t), self.Mt, self.Wt / self.Mt,
+                 dptr(u), dptr(work), int(nbytes[0]), stream_ptr())
+            return u
+        d_t = _dev(t)
+        call("vtb_reconstruct_workspace", N, len(t), self.Mt, nbytes.ctypes.data)
+        work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device="cuda")
         call("vtb_reconstruct", dptr(dirich), N, Py * Px, dptr(tk1), dptr(tk2), dptr(c), dptr(ind),
              dptr(self.d_norm), self.size, dptr(d_t), len(t), self.Mt, self.Wt / self.Mt, dptr(u), dptr(work),
              int(nbytes[0]), stream_ptr())
