@@ -1,9 +1,8 @@
-// FP64 register-tiled GEMM on the CUDA cores (DFMA), used by the plain
-// float64 path: C[m, n] = alpha * sum_k A(m, k) B(n, k) + beta * C[m, n]
+// FP64 GEMM on the float64 tensor-core path, used by the plain float64
+// path: C[m, n] = alpha * sum_k A(m, k) B(n, k) + beta * C[m, n]
 // with arbitrary element strides, so one kernel serves the RF projection
 // (video x RFs), the synthesis (H x spatial functions) and the small
-// cross-weight products.  64x64 output tile per 256-thread block, 4x4 per
-// thread, k staged through shared memory in slabs of 16.
+// cross-weight products.
 #pragma once
 #include "common.cuh"
 
