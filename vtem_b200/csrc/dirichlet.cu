@@ -4,9 +4,8 @@
 //      restricted to the spatial ellipse (compute_Ds + fft2Ds_kernel,
 //      vtem/vrf.py:333-377, :1293-1350).  Only (2Mx+1)(2My+1) of the
 //      LPy*LPx frequencies are ever used, so instead of a full 2-D FFT the
-//      kernel evaluates a separable DFT for just those bins: rows are staged
-//      through shared memory 16 at a time and reduced against an exact
-//      twiddle table (sincospi of integer ratios), one block per RF.
+//      kernels evaluate a separable DFT for just those bins against exact
+//      twiddle tables (sincospi of integer ratios).
 //  vtb_dirich_space : phi_n on the decode grid, equal to the reference's
 //      unnormalised inverse FFT on the (Py1, Px1) period grid followed by the
 //      centred crop (compute_dirich_space_fft, vrf.py:437-499, :585-677),
@@ -16,6 +15,8 @@
 //  vtb_compute_q : compute_q_Kernel (vtem/dirichlet.py:204-222).
 //  vtb_compute_G : compute_G_Kernel + diag_add_Kernel (dirichlet.py:272-350),
 //      the same entries as products of the intervals' harmonics.
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_f64.cuh"
 
@@ -23,8 +24,166 @@ namespace vtb {
 
 // ---------------------------------------------------------------- Ds (DFT)
 
+// The same coefficients on the float64 tensor path, for up to 16 bins each way
+// (2Mx+1, 2My+1 <= 16).  An RF is real, so the bins of +-m are the sums with
+// cos and sin of |m|: 2M+1 real columns each way, at most 16.  A block takes
+// one RF at a time (persistent over the RFs, the cos/sin tables formed once):
+//   R = RF (rows x px) * X (px x 16): a warp per 16 rows, the RF's fragments
+//       straight from global memory (whole sectors, read once), X from shared
+//       memory;
+//   S = Y^T (16 x rows) * R: the rows split over the warps, the partial sums
+//       added in warp order;
+// then the four real sums of each |my|, |mx| give its (up to) four bins.
+// Bound: the HBM read of the RFs (537 MB at 1024 RFs of 256 x 256, 82 us).
+// A lane's fragment holds the pixels 2q and 2q + 1 of a step's eight (16-byte
+// loads where rows allow), so both products take k in that order.  Measured at
+// that size: 2306 us with a dot product per bin and row, 125 here.
+constexpr int kDfWarps = 8;
+constexpr int kDfS = 18;        // row stride of tables and R: fragment reads free of bank conflicts
+
+__device__ __forceinline__ void df_mma(double (&c)[4], double a0, double a1, double b) {
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a0), "d"(a1), "d"(b));
+}
+
+// t[p * kDfS + col]: col 0 = 1, 2b - 1 = cos(2 pi b p / L), 2b = sin(2 pi b p / L), b <= M; zero elsewhere
+__device__ void df_table(int L, int Lpad, int M, double* __restrict__ t) {
+    for (int e = threadIdx.x; e < Lpad * 9; e += blockDim.x) {
+        const int p = e / 9, b = e % 9;
+        double s = 0.0, c = 0.0;
+        if (p < L && b <= M) sincospi(2.0 * (double)(((int64_t)b * p) % L) / L, &s, &c);
+        if (b == 0) {
+            t[p * kDfS] = c;
+        } else if (b < 8) {
+            t[p * kDfS + 2 * b - 1] = c;
+            t[p * kDfS + 2 * b] = s;
+        } else {
+            t[p * kDfS + 15] = 0.0;
+        }
+    }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kDfWarps * 32) ds_mma_kernel(const double* __restrict__ rf, int64_t rf_ld, int N,
+                                                               int LPy, int LPx, int Mx, int My, double dxdy,
+                                                               double2* __restrict__ Ds) {
+    extern __shared__ double dsm[];
+    const int Xp = (LPx + 7) & ~7, Yp = (LPy + 15) & ~15;
+    double* R = dsm;                               // Yp x kDfS
+    double* ty = R + (size_t)Yp * kDfS;            // Yp x kDfS
+    double* tx = LPx == LPy && Mx == My ? ty : ty + (size_t)Yp * kDfS;   // Xp x kDfS
+    __shared__ double part[kDfWarps][16 * 16];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int fr = lane >> 2, fq = lane & 3;
+    df_table(LPy, Yp, My, ty);
+    if (tx != ty) df_table(LPx, Xp, Mx, tx);
+    const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
+    for (int n = blockIdx.x; n < N; n += gridDim.x) {
+        __syncthreads();                           // tables formed; the last RF's sums have been read
+        const double* src = rf + (int64_t)n * rf_ld;
+        for (int r0 = 16 * w; r0 < Yp; r0 += 16 * kDfWarps) {
+            double acc[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) acc[j][h] = 0.0;
+            const bool in0 = r0 + fr < LPy, in1 = r0 + fr + 8 < LPy;
+            const double* p0 = src + (int64_t)(in0 ? r0 + fr : 0) * LPx + 2 * fq;
+            const double* p1 = src + (int64_t)(in1 ? r0 + fr + 8 : 0) * LPx + 2 * fq;
+            constexpr int kU = 4;                  // steps of eight pixels whose loads are issued together
+            for (int x0 = 0; x0 < Xp; x0 += 8 * kU) {
+                double2 v0[kU], v1[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const int x = x0 + 8 * u, c = x + 2 * fq;
+                    v0[u] = v1[u] = make_double2(0.0, 0.0);
+                    if (VEC) {                     // LPx even: a pair is whole or outside
+                        if (c < LPx) {
+                            if (in0) v0[u] = __ldcs(reinterpret_cast<const double2*>(p0 + x));
+                            if (in1) v1[u] = __ldcs(reinterpret_cast<const double2*>(p1 + x));
+                        }
+                    } else {
+                        if (c < LPx) {
+                            if (in0) v0[u].x = __ldcs(p0 + x);
+                            if (in1) v1[u].x = __ldcs(p1 + x);
+                        }
+                        if (c + 1 < LPx) {
+                            if (in0) v0[u].y = __ldcs(p0 + x + 1);
+                            if (in1) v1[u].y = __ldcs(p1 + x + 1);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const int x = x0 + 8 * u;
+                    if (x >= Xp) break;
+                    const double* t = tx + (size_t)(x + 2 * fq) * kDfS + fr;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        df_mma(acc[j], v0[u].x, v1[u].x, t[8 * j]);
+                        df_mma(acc[j], v0[u].y, v1[u].y, t[kDfS + 8 * j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    R[(size_t)(r0 + fr + 8 * (h >> 1)) * kDfS + 8 * j + 2 * fq + (h & 1)] = acc[j][h];
+        }
+        __syncthreads();
+        {
+            double acc[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) acc[j][h] = 0.0;
+            for (int y = 8 * w; y < Yp; y += 8 * kDfWarps) {
+                const double* t = ty + (size_t)(y + 2 * fq) * kDfS + fr;
+                const double* r = R + (size_t)(y + 2 * fq) * kDfS + fr;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    df_mma(acc[j], t[0], t[8], r[8 * j]);
+                    df_mma(acc[j], t[kDfS], t[kDfS + 8], r[kDfS + 8 * j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    part[w][(fr + 8 * (h >> 1)) * 16 + 8 * j + 2 * fq + (h & 1)] = acc[j][h];
+        }
+        __syncthreads();
+        {
+            double v = part[0][tid];
+#pragma unroll
+            for (int k = 1; k < kDfWarps; ++k) v += part[k][tid];
+            part[0][tid] = v;
+        }
+        __syncthreads();
+        if (tid < Kx * Ky) {
+            const int mx = tid % Kx - Mx, my = My - tid / Kx;      // storage row holds my = My - row
+            double2 out = make_double2(0.0, 0.0);
+            if ((int64_t)mx * mx * My * My + (int64_t)my * my * Mx * Mx <= (int64_t)Mx * Mx * My * My) {
+                const int b = abs(mx), a = abs(my);
+                const int rc = a ? 2 * a - 1 : 0, cc = b ? 2 * b - 1 : 0;
+                const double* S = part[0];
+                const double Cc = S[rc * 16 + cc];
+                const double Sc = a ? S[(rc + 1) * 16 + cc] : 0.0, Cs = b ? S[rc * 16 + cc + 1] : 0.0;
+                const double Ss = a && b ? S[(rc + 1) * 16 + cc + 1] : 0.0;
+                const double ya = my < 0 ? -1.0 : 1.0, xb = mx < 0 ? -1.0 : 1.0;
+                const double sgn = ((mx + my) % 2 == 0) ? dxdy : -dxdy;
+                out = make_double2(sgn * (Cc - ya * xb * Ss), -sgn * (ya * Sc + xb * Cs));
+            }
+            Ds[(int64_t)n * Kx * Ky + tid] = out;
+        }
+    }
+}
+
 constexpr int kDsRows = 16;
 
+// Any bin count (2Mx+1)(2My+1) <= 256: a dot product per bin and row.
 __global__ void __launch_bounds__(256) ds_kernel(const double* __restrict__ rf, int64_t rf_ld, int LPy, int LPx,
                                                   int Mx, int My, double dxdy, double2* __restrict__ Ds) {
     extern __shared__ double smem[];
@@ -96,49 +255,78 @@ __global__ void __launch_bounds__(256) ds_kernel(const double* __restrict__ rf, 
 
 // ---------------------------------------------------------------- phi
 
+// Thread = a pixel column and four rows of it at a time: a spectral column
+// sum Q read from shared memory serves four pixels.  The twiddles of the
+// period (exact integer reductions) are formed once per block, not per term.
+// Measured at 1024 RFs, 64 x 64, Mx = My = 6: 150 us with a sincospi per term,
+// 52 here.
+constexpr int kPhiRows = 4;
+
 __global__ void __launch_bounds__(256) dirich_space_kernel(const double2* __restrict__ Ds, int Mx, int My, int Px,
-                                                            int Py, int Px1, int Py1, double* __restrict__ out) {
+                                                            int Py, int Px1, int Py1, int table,
+                                                            double* __restrict__ out) {
     extern __shared__ double smem[];
     const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
     double2* Q = reinterpret_cast<double2*>(smem);  // Ky x Px : sum over mx
     double2* ey = Q + Ky * Px;                       // Ky x Py
+    double2* tw = ey + Ky * Py;                      // e^{2 pi i r / Px1}, r < Px1 (when table)
     const int n = blockIdx.x;
     const int tid = threadIdx.x;
     const int xd = (Px1 - Px) / 2, yd = (Py1 - Py) / 2;
     const double2* D = Ds + (int64_t)n * Kx * Ky;
+    auto twiddle = [](int r, int L) {
+        double s, c;
+        sincospi(2.0 * r / L, &s, &c);
+        return make_double2(c, s);
+    };
+    if (table) {
+        for (int r = tid; r < Px1; r += blockDim.x) tw[r] = twiddle(r, Px1);
+        __syncthreads();
+    }
     for (int o = tid; o < Ky * Px; o += blockDim.x) {
         const int myi = o / Px, px = o % Px;
         const int my = myi - My;
         double sr = 0.0, si = 0.0;
+        int r = (int)((((int64_t)-Mx * (px + xd)) % Px1 + Px1) % Px1);   // mx (px + xd) mod Px1
+        const int step = (px + xd) % Px1;
         for (int mx = -Mx; mx <= Mx; ++mx) {
             const double2 d = D[(My - my) * Kx + (mx + Mx)];
             const double sg = (((mx + my) % 2) == 0) ? 1.0 : -1.0;
-            const int64_t r = ((((int64_t)mx * (px + xd)) % Px1) + Px1) % Px1;
-            double s, c;
-            sincospi(2.0 * r / Px1, &s, &c);
-            sr += sg * (d.x * c - d.y * s);
-            si += sg * (d.x * s + d.y * c);
+            const double2 e = table ? tw[r] : twiddle(r, Px1);
+            sr += sg * (d.x * e.x - d.y * e.y);
+            si += sg * (d.x * e.y + d.y * e.x);
+            r += step;
+            if (r >= Px1) r -= Px1;
         }
         Q[o] = make_double2(sr, si);
     }
     for (int o = tid; o < Ky * Py; o += blockDim.x) {
         const int myi = o / Py, py = o % Py;
         const int my = myi - My;
-        const int64_t r = ((((int64_t)my * (py + yd)) % Py1) + Py1) % Py1;
-        double s, c;
-        sincospi(2.0 * r / Py1, &s, &c);
-        ey[o] = make_double2(c, s);
+        ey[o] = twiddle((int)(((((int64_t)my * (py + yd)) % Py1) + Py1) % Py1), Py1);
     }
     __syncthreads();
-    for (int p = tid; p < Px * Py; p += blockDim.x) {
-        const int py = p / Px, px = p % Px;
-        double acc = 0.0;
+    const int groups = (Py + kPhiRows - 1) / kPhiRows;
+    for (int p = tid; p < Px * groups; p += blockDim.x) {
+        const int py = (p / Px) * kPhiRows, px = p % Px;
+        double acc[kPhiRows];
+        int row[kPhiRows];
+#pragma unroll
+        for (int i = 0; i < kPhiRows; ++i) {
+            acc[i] = 0.0;
+            row[i] = min(py + i, Py - 1);
+        }
         for (int myi = 0; myi < Ky; ++myi) {
             const double2 q = Q[myi * Px + px];
-            const double2 e = ey[myi * Py + py];
-            acc = fma(q.x, e.x, fma(-q.y, e.y, acc));
+#pragma unroll
+            for (int i = 0; i < kPhiRows; ++i) {
+                const double2 e = ey[myi * Py + row[i]];
+                acc[i] = fma(q.x, e.x, fma(-q.y, e.y, acc[i]));
+            }
         }
-        out[(int64_t)n * Px * Py + p] = acc;
+#pragma unroll
+        for (int i = 0; i < kPhiRows; ++i)
+            if (py + i < Py) out[(int64_t)n * Px * Py + (int64_t)(py + i) * Px + px] = acc[i];
     }
 }
 
@@ -406,6 +594,19 @@ VTB_API int vtb_dirichlet_coeffs(const double* rf, int N, int LPy, int LPx, int6
     VTB_CHECK_ARG(rf && Ds);
     const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
     VTB_CHECK_ARG(Kx * Ky <= 256);
+    // the tensor path needs its tables and one RF's row sums in shared memory
+    // (256 x 256: 74 KB, three blocks per SM); longer sides and more bins take the general kernel
+    const int Xp = (LPx + 7) & ~7, Yp = (LPy + 15) & ~15;
+    const size_t smm = (size_t)(2 * Yp + (LPx == LPy && Mx == My ? 0 : Xp)) * kDfS * sizeof(double);
+    if (Kx <= 16 && Ky <= 16 && smm <= 200 * 1024) {
+        const bool vec = LPx % 2 == 0 && rf_ld % 2 == 0 && ((uintptr_t)rf & 15) == 0;
+        auto kernel = vec ? ds_mma_kernel<true> : ds_mma_kernel<false>;
+        VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
+        const int per_sm = smm > 100 * 1024 ? 1 : smm > 56 * 1024 ? 2 : 4;
+        kernel<<<std::min(N, per_sm * kNumSMs), kDfWarps * 32, smm, as_stream(stream)>>>(
+            rf, rf_ld, N, LPy, LPx, Mx, My, dxdy, reinterpret_cast<double2*>(Ds));
+        return launch_status();
+    }
     const size_t sm = (size_t)(LPx + LPy) * sizeof(double2) + (size_t)kDsRows * LPx * sizeof(double) +
                       (size_t)kDsRows * Kx * sizeof(double2);
     VTB_CHECK_ARG(sm <= 200 * 1024);
@@ -424,13 +625,15 @@ VTB_API int vtb_dirich_space(const double* Ds, int N, int Mx, int My, int Px, in
     if (N == 0) return VTB_OK;
     VTB_CHECK_ARG(Ds && out);
     const int Ky = 2 * My + 1;
-    const size_t sm = (size_t)Ky * (Px + Py) * sizeof(double2);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
+    const size_t base = (size_t)Ky * (Px + Py) * sizeof(double2);
+    VTB_CHECK_ARG(base <= 200 * 1024);
+    const int table = base + (size_t)Px1 * sizeof(double2) <= 200 * 1024;
+    const size_t sm = base + (table ? (size_t)Px1 * sizeof(double2) : 0);
     if (sm > 48 * 1024)
         VTB_CUDA_TRY(
             cudaFuncSetAttribute(dirich_space_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     dirich_space_kernel<<<N, 256, sm, as_stream(stream)>>>(reinterpret_cast<const double2*>(Ds), Mx, My, Px, Py,
-                                                          Px1, Py1, out);
+                                                          Px1, Py1, table, out);
     return launch_status();
 }
 
