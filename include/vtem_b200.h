@@ -545,6 +545,14 @@ int vtb_sym_pinv_batched(double* M, const double* b, double* x, int K, int batch
 int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double* x, double* x_tmp, int K, double dt_alpha,
                   int steps, void* bar, void* stream);
 
+/* The same iterate as vtb_rnn_coeff for symmetric Mr, by repeated squaring of
+ * the update's map (a few float64 products in place of most of the exchanges
+ * between SMs), all scratch in one workspace (256-byte aligned),
+ * which begins with vtb_rnn_coeff's status words.  The form the decoder uses. */
+int vtb_rnn_coeff_workspace(int K, int64_t* bytes);
+int vtb_rnn_coeff_work(const double* Mr, int64_t ld, const double* br, double* x, int K, double dt_alpha, int steps,
+                       void* work, int64_t work_bytes, void* stream);
+
 /* out (device) = ||dx|| / ||x||: the relative size of a refinement correction. */
 int vtb_norm_ratio(const double* dx, const double* x, int n, double* out, void* stream);
 /* y += x (n doubles). */

@@ -96,6 +96,8 @@ SIGNATURES = {
     "vtb_sym_pinv_batched_workspace": [I, I, P],
     "vtb_sym_pinv_batched": [P, P, P, I, I, D, P, L, P, P, P],
     "vtb_rnn_coeff": [P, L, P, P, P, I, D, I, P, P],
+    "vtb_rnn_coeff_workspace": [I, P],
+    "vtb_rnn_coeff_work": [P, L, P, P, I, D, I, P, L, P],
     "vtb_tc_group_bytes": [I],  # restype int64, set in lib()
     "vtb_tc_group_build": [P, I, P, P, P, P, P, P, P, P, I, P],
     "vtb_tc_gemm_grouped": [P, I, I, I, P],

@@ -38,6 +38,11 @@ __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, doubl
         : "d"(a0), "d"(a1), "d"(b));
 }
 
+// How a kernel uses its grid: one CTA a tile; a cluster of gridDim.z CTAs
+// sharing a tile's k range; or C = A A^T + beta A (A square and symmetric),
+// the tiles of the lower triangle computed and written twice.
+enum { kWhole = 0, kSplit = 1, kSym = 2 };
+
 // One operand's slab: ROWS x kBK, KF: k fastest.  V doubles a copy.
 template <int ROWS, bool KF, int V>
 struct Slab {
@@ -86,8 +91,10 @@ struct Slab {
     }
 };
 
-template <int BM, int BN, int WR, int WC, int ST, bool AKF, bool BKF, int V, bool SPLIT>
+template <int BM, int BN, int WR, int WC, int ST, bool AKF, bool BKF, int V, int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p) {
+    constexpr bool SPLIT = MODE == kSplit;
+    if (MODE == kSym && blockIdx.x > blockIdx.y) return;   // the mirror of a tile below the diagonal
     using SA = Slab<BM, AKF, V>;
     using SB = Slab<BN, BKF, V>;
     constexpr int MT = BM / WR / 16, NT = BN / WC / 8;
@@ -102,13 +109,17 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p
     const int slabs = (p.K + kBK - 1) / kBK, splits = SPLIT ? gridDim.z : 1;
     const int k_lo = SPLIT ? (int)((int64_t)slabs * blockIdx.z / splits) : 0;
     const int nk = SPLIT ? (int)((int64_t)slabs * (blockIdx.z + 1) / splits) : slabs;
-    double acc[MT][NT][4];
+    const int fr = lane >> 2, fk = lane & 3;
+    double acc[MT][NT][4];   // (C = A^2 + beta A: the addend first, so that the sum is one chain of FMAs)
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
+            for (int h = 0; h < 4; ++h) {
+                const int gm = m0 + wm + 16 * i + 8 * (h >> 1) + fr, gn = n0 + wn + 8 * j + 2 * fk + (h & 1);
+                acc[i][j][h] = MODE == kSym && gm < p.M && gn < p.N ? p.beta * p.A[(int64_t)gm * p.a_m + gn] : 0.0;
+            }
     SA la;
     SB lb;
     la.init(p.A, p.a_m, p.a_k, m0, k_lo * kBK, p.M);
@@ -122,7 +133,6 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p
     };
     for (int s = 0; s < ST - 1; ++s) load(k_lo + s, s);
     int cur = 0, nxt = ST - 1;   // the ring's places of the slab in use and of the next to be issued
-    const int fr = lane >> 2, fk = lane & 3;
     for (int kb = k_lo; kb < nk; ++kb) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
         __syncthreads();   // slab kb has arrived for every thread; slab kb - 1 has been read by every warp
@@ -159,8 +169,17 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int h = 0; h < 4; ++h)
-                    store(m0 + wm + 16 * i + 8 * (h >> 1) + fr, n0 + wn + 8 * j + 2 * fk + (h & 1), acc[i][j][h]);
+                for (int h = 0; h < 4; ++h) {
+                    const int gm = m0 + wm + 16 * i + 8 * (h >> 1) + fr, gn = n0 + wn + 8 * j + 2 * fk + (h & 1);
+                    if constexpr (MODE == kSym) {
+                        if (gm >= p.M || gn >= p.N) continue;
+                        const double v = acc[i][j][h];
+                        p.C[(int64_t)gm * p.c_m + gn] = v;
+                        if (m0 != n0) p.C[(int64_t)gn * p.c_m + gm] = v;
+                    } else {
+                        store(gm, gn, acc[i][j][h]);
+                    }
+                }
     } else {
         // the cluster's partial tiles, each in its CTA's shared memory, added in
         // rank order; CTA r takes the r-th part of the tile, consecutive threads
@@ -193,8 +212,8 @@ template <int BM, int BN, int WR, int WC, int ST, bool AKF, bool BKF, int V>
 static int launch_tile(const GemmF64Args& p, int splits, cudaStream_t s) {
     constexpr size_t sm = (size_t)ST * (Slab<BM, AKF, V>::kDoubles + Slab<BN, BKF, V>::kDoubles) * sizeof(double);
     static_assert(sm >= BM * (BN + 1) * sizeof(double), "a partial tile fits the slabs");
-    auto kernel = splits > 1 ? gemm_f64_kernel<BM, BN, WR, WC, ST, AKF, BKF, V, true>
-                             : gemm_f64_kernel<BM, BN, WR, WC, ST, AKF, BKF, V, false>;
+    auto kernel = splits > 1 ? gemm_f64_kernel<BM, BN, WR, WC, ST, AKF, BKF, V, kSplit>
+                             : gemm_f64_kernel<BM, BN, WR, WC, ST, AKF, BKF, V, kWhole>;
     VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ceil_div(p.N, BN), ceil_div(p.M, BM), splits);
@@ -256,6 +275,28 @@ int gemm_f64(const GemmF64Args& p, cudaStream_t s) {
     if (akf) return v2 ? launch_layout<true, false, 2>(p, s) : launch_layout<true, false, 1>(p, s);
     if (bkf) return v2 ? launch_layout<false, true, 2>(p, s) : launch_layout<false, true, 1>(p, s);
     return v2 ? launch_layout<false, false, 2>(p, s) : launch_layout<false, false, 1>(p, s);
+}
+
+template <int T, int ST, int V>
+static int launch_sym(const GemmF64Args& p, cudaStream_t s) {
+    constexpr size_t sm = (size_t)2 * ST * Slab<T, true, V>::kDoubles * sizeof(double);
+    auto kernel = gemm_f64_kernel<T, T, 2, 2, ST, true, true, V, kSym>;
+    VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    kernel<<<dim3(ceil_div(p.N, T), ceil_div(p.M, T)), kGemmThreads, sm, s>>>(p);
+    return launch_status();
+}
+
+int square_f64(int N, const double* A, int64_t lda, double beta, double* C, int64_t ldc, cudaStream_t s) {
+    if (N <= 0) return VTB_OK;
+    if (ceil_div(N, 32) > 65535) return VTB_BAD_ARG;
+    const GemmF64Args p{N, N, N, A, lda, 1, A, lda, 1, C, ldc, 1, 1.0, beta};
+    const bool v2 = lda % 2 == 0 && ((uintptr_t)A & 15) == 0;
+    // 64 x 64 tiles come three CTAs to an SM in waves of 444; up to a few waves
+    // the ragged last one costs more than the small tiles' operand traffic
+    // (N = K = 1921, 496 tiles: 384 us; 1891 tiles of 32 x 32: 285 us)
+    const int64_t t = ceil_div(N, 64);
+    if (t * (t + 1) / 2 < 12 * kNumSMs) return v2 ? launch_sym<32, 4, 2>(p, s) : launch_sym<32, 4, 1>(p, s);
+    return v2 ? launch_sym<64, 3, 2>(p, s) : launch_sym<64, 3, 1>(p, s);
 }
 
 }  // namespace vtb

@@ -22,4 +22,8 @@ struct GemmF64Args {
 // C(m, n) = alpha sum_k A(m, k) B(n, k) + beta C(m, n) on `s` (gemm_f64.cu).
 int gemm_f64(const GemmF64Args& p, cudaStream_t s);
 
+// C = A^2 + beta A for symmetric A (N x N, rows of lda doubles), C exactly
+// symmetric: the tiles of one triangle computed, written to both (gemm_f64.cu).
+int square_f64(int N, const double* A, int64_t lda, double beta, double* C, int64_t ldc, cudaStream_t s);
+
 }  // namespace vtb

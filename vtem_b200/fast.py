@@ -468,12 +468,14 @@ class CoeffDecoder(object):
         self._build_real(s)
         if dt_alpha is None:
             dt_alpha = 1.0 / self.lambda_max()
-        bar = torch.zeros(4, dtype=torch.int32, device=dev)
-        call("vtb_rnn_coeff", dptr(self.Mr), self.K, dptr(self.br), dptr(self.xr), dptr(self.rr), self.K,
-             float(dt_alpha), int(steps), dptr(bar), s)
+        nb = np.zeros(1, np.int64)
+        call("vtb_rnn_coeff_workspace", self.K, nb.ctypes.data)
+        work = torch.empty(int(nb[0]), dtype=torch.uint8, device=dev)
+        call("vtb_rnn_coeff_work", dptr(self.Mr), self.K, dptr(self.br), dptr(self.xr), self.K, float(dt_alpha),
+             int(steps), dptr(work), work.numel(), s)
         call("vtb_coeff_unrealify_vec", dptr(self.xr), self.K, 1, dptr(self.a), 0, s)
-        if int(bar[2].item()) != 0:
-            raise VtbError("vtb_rnn_coeff", _abi.VTB_TIMEOUT)
+        if int(work[:16].view(torch.int32)[2].item()) != 0:
+            raise VtbError("vtb_rnn_coeff_work", _abi.VTB_TIMEOUT)
         self.last_solver = "rnn"
         return self.a, float(dt_alpha)
 
