@@ -15,7 +15,7 @@
 //   b[(s,m)]         = sum_n d_n[s] g_n[m],  g_n[m] = sum_{k in n} conj(T_k(m)) q_k,
 // so Phi (n x K) is never formed: one pass over the spikes builds W_n, g_n
 // (temporal_gram_kernel), one tiled pass over the neurons builds M
-// (kron_gram_kernel).  The synthesis expands a on the separable
+// (kron_gram.cu).  The synthesis expands a on the separable
 // space-time basis: A[t, s] = sum_m a[s, m] e^{jmWt}, then per frame
 // u = Re(ey^T A_t ex) on the decode grid (synth_kernel), whose output write is
 // the one HBM-sized stream of the whole decode.
@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "kron_gram.cuh"
 
 namespace vtb {
 
@@ -305,75 +306,6 @@ __global__ void __launch_bounds__(kNrWarps * 32) coeff_residual_warp_kernel(
         }
     }
     if (lane < Kt) gres[(int64_t)nr * Kt + lane] = gacc;
-}
-
-// ------------------------------------------------------------------ M
-// Block = 4 x 4 tile of (s, s') pairs (s-tile <= s'-tile: M is Hermitian and
-// the mirror half is written from the same accumulators); threads own (m, m')
-// entries of the Kt x Kt sub-blocks.  d products for a chunk of neurons are
-// staged in shared memory; W_n entries stream from L2, coalesced.
-constexpr int kKT = 4;
-constexpr int kKN = 32;
-
-__global__ void __launch_bounds__(256) kron_gram_kernel(const double2* __restrict__ d, int N, int Ks,
-                                                        const double2* __restrict__ Wn, int Kt,
-                                                        double2* __restrict__ M, int64_t ldm) {
-    __shared__ double2 sa[kKN][kKT * kKT];
-    // map blockIdx.x to an upper-triangular tile pair (ti <= tj)
-    const int T = (Ks + kKT - 1) / kKT;
-    int b = blockIdx.x, ti = 0;
-    while (b >= T - ti) { b -= T - ti; ++ti; }
-    const int tj = ti + b;
-    const int s0 = ti * kKT, s1 = tj * kKT;
-    const int KK = Kt * Kt;
-    for (int e0 = 0; e0 < KK; e0 += blockDim.x) {
-        const int e = e0 + threadIdx.x;
-        double2 acc[kKT][kKT];
-#pragma unroll
-        for (int i = 0; i < kKT; ++i)
-#pragma unroll
-            for (int j = 0; j < kKT; ++j) acc[i][j] = make_double2(0, 0);
-        for (int n0 = 0; n0 < N; n0 += kKN) {
-            const int nn = min(kKN, N - n0);
-            __syncthreads();
-            for (int x = threadIdx.x; x < nn * kKT * kKT; x += blockDim.x) {
-                const int r = x / (kKT * kKT), ij = x % (kKT * kKT), i = ij / kKT, j = ij % kKT;
-                const int si = s0 + i, sj = s1 + j;
-                double2 v = make_double2(0, 0);
-                if (si < Ks && sj < Ks) v = cmulc(d[(int64_t)(n0 + r) * Ks + si], d[(int64_t)(n0 + r) * Ks + sj]);
-                sa[r][ij] = v;
-            }
-            __syncthreads();
-            if (e < KK) {
-                double2 wnext = Wn[(int64_t)n0 * KK + e];
-                for (int r = 0; r < nn; ++r) {
-                    const double2 w = wnext;
-                    if (r + 1 < nn) wnext = Wn[(int64_t)(n0 + r + 1) * KK + e];
-#pragma unroll
-                    for (int i = 0; i < kKT; ++i)
-#pragma unroll
-                        for (int j = 0; j < kKT; ++j) {
-                            const double2 a = sa[r][i * kKT + j];
-                            acc[i][j].x = fma(a.x, w.x, fma(-a.y, w.y, acc[i][j].x));
-                            acc[i][j].y = fma(a.x, w.y, fma(a.y, w.x, acc[i][j].y));
-                        }
-                }
-            }
-        }
-        if (e < KK) {
-            const int m = e / Kt, mp = e % Kt;
-#pragma unroll
-            for (int i = 0; i < kKT; ++i)
-#pragma unroll
-                for (int j = 0; j < kKT; ++j) {
-                    const int si = s0 + i, sj = s1 + j;
-                    if (si >= Ks || sj >= Ks) continue;
-                    const int64_t row = (int64_t)si * Kt + m, col = (int64_t)sj * Kt + mp;
-                    M[col * ldm + row] = acc[i][j];  // column-major
-                    if (ti != tj) M[row * ldm + col] = make_double2(acc[i][j].x, -acc[i][j].y);
-                }
-        }
-    }
 }
 
 // b[(s, m)] = sum_n d[n][s] g[n][m]: a cluster of kRhsSplit CTAs per group
@@ -1086,12 +1018,8 @@ VTB_API int vtb_coeff_pack(const double* Ds, int N, int Kfull, const int32_t* sm
 VTB_API int vtb_coeff_gram(const double* d, int N, int Ks, const double* Wn, const double* gn, int Kt, double* M,
                            int64_t ldm, double* b, void* stream) {
     VTB_CHECK_ARG(N > 0 && Ks > 0 && Kt > 0 && d && Wn && gn && M && b && ldm >= (int64_t)Ks * Kt);
-    const int T = (Ks + kKT - 1) / kKT;
-    const int tiles = T * (T + 1) / 2;
-    kron_gram_kernel<<<tiles, 256, 0, as_stream(stream)>>>(reinterpret_cast<const double2*>(d), N, Ks,
-                                                           reinterpret_cast<const double2*>(Wn), Kt,
-                                                           reinterpret_cast<double2*>(M), ldm);
-    int st = launch_status();
+    int st = kron_gram_f64(reinterpret_cast<const double2*>(d), N, Ks, reinterpret_cast<const double2*>(Wn), Kt,
+                           reinterpret_cast<double2*>(M), ldm, as_stream(stream));
     if (st) return st;
     kron_rhs_kernel<<<rhs_grid(Ks), 256, rhs_smem(Kt), as_stream(stream)>>>(
         reinterpret_cast<const double2*>(d), N, Ks, reinterpret_cast<const double2*>(gn), Kt,
