@@ -492,6 +492,31 @@ int vtb_chol_factor_inverse(float* A, int64_t ld, int K, float* Dinv, float* Lin
  * Replaces spotrs in the solve of linalg.py:591-631. */
 int64_t vtb_chol_solve_inverse_bytes(int K);
 int vtb_chol_solve_inverse(const float* Linv, int K, double* x, void* work, int64_t work_bytes, void* stream);
+
+/* Batches of vtb_chol_factor_inverse / vtb_chol_solve_inverse: systems of any
+ * sizes, one launch each.  vtb_chol_batch_build fills `host`
+ * (vtb_chol_batch_bytes(n) bytes, then copied to the device by the caller)
+ * from host arrays of the systems' device addresses; work is the device
+ * buffer of vtb_chol_batch_work_bytes bytes (256-byte aligned) they share,
+ * *grid the CTAs of the launch.  The status words are cleared by the caller
+ * before every vtb_chol_batch_factor.  vtb_chol_batch_solve works in place on
+ * x[which] of every descriptor (an array in device memory; tile0 counts the
+ * ceil(K/64)(ceil(K/64)+1)/2 tiles of the systems before, `tiles` all of them;
+ * work as in vtb_chol_solve_inverse). */
+typedef struct {
+    const float* Linv;
+    float* work;
+    double* x[2];
+    int64_t reserved;
+    int32_t K, tile0;
+} vtb_inv_system;
+int64_t vtb_chol_batch_bytes(int n);
+int vtb_chol_batch_work_bytes(int n, const int32_t* K, int64_t* bytes);
+int vtb_chol_batch_build(void* host, int n, const uint64_t* A, const int64_t* ld, const int32_t* K,
+                         const uint64_t* Dinv, const uint64_t* Linv, uint64_t work, const uint64_t* status,
+                         const uint64_t* pivots, const double* rcond, int32_t* grid);
+int vtb_chol_batch_factor(const void* desc, int n, int grid, void* work, int64_t work_bytes, void* stream);
+int vtb_chol_batch_solve(const vtb_inv_system* systems, int n, int tiles, int which, void* stream);
 /* Pseudoinverse solve x = V diag(1/w if |w| > rcond*max|w| else 0) V^T b of
  * a float64 symmetric M (destroyed), the rule of solve_eq_sym
  * (vtem/utils/linalg.py:591-631, sq_Kernel :791-833).  kept (device) the

@@ -9,12 +9,12 @@ batch changes how the work is scheduled:
   round-robin on several CUDA streams; the tensor-core Kronecker Grams of all
   clips run as ONE grouped GEMM launch (``GroupedGram``, tile width chosen by
   timing), then each is scattered into its real symmetric float32 system;
-* clips whose systems have the same size K are factorised by one batched
-  float32 Cholesky per group (``vtb_sym_factor_batched``), and every clip's
-  triangular solves run in one launch (``vtb_sym_potrs_batched``, one CTA per
-  clip), the grouped counterpart of the reference's per-window solve
-  (vtem/vtdm.py:645-648); float64 refinement sweeps against each clip's
-  exact residual follow;
+* every clip's system is factorised and its factor inverted in one launch
+  (``vtb_chol_batch_factor``: teams of CTAs, each running the tile Cholesky of
+  its clips), and every clip's solves are two products in two launches
+  (``vtb_chol_batch_solve``), the grouped counterpart of the reference's
+  per-window solve (vtem/vtdm.py:645-648); float64 refinement sweeps against
+  each clip's exact residual follow;
 * that whole sequence, up to the acceptance check, is captured once as a
   CUDA graph and replayed per run (``graph=True``);
 * one host check then reads every clip's flags: a clip whose pseudoinverse
@@ -40,7 +40,8 @@ import torch
 from . import autotune, fast
 from ._abi import call, dptr, lib, stream_ptr
 
-TRSV_DESC = np.dtype([("L", "<u8"), ("Dinv", "<u8"), ("x", "<u8"), ("ld", "<i8"), ("K", "<i4"), ("pad", "<i4")])
+INV_SYSTEM = np.dtype([("Linv", "<u8"), ("work", "<u8"), ("x", "<u8", 2), ("reserved", "<i8"), ("K", "<i4"),
+                       ("tile0", "<i4")])
 
 
 class ClipProblem(object):
@@ -172,17 +173,9 @@ def sweep_update(d, i, s):
     call("vtb_daxpy1", dptr(d.xr), dptr(d.rr), d.K, s)
 
 
-def trsv_descs(entries, device):
-    """Device array of vtb_trsv_desc for (L, Dinv, x, ld, K) tuples."""
-    a = np.zeros(len(entries), TRSV_DESC)
-    for i, (L, Dinv, x, ld, K) in enumerate(entries):
-        a[i] = (L, Dinv, x, ld, K, 0)
-    return torch.as_tensor(np.frombuffer(a.tobytes(), np.uint8).copy()).to(device)
-
-
 class MixedSolvePlan(object):
-    """Grouped float32 Cholesky, batched triangular solves and float64
-    refinement sweeps of a set of mixed decoders whose systems were staged by
+    """Batched float32 Cholesky with inverses, batched product solves and
+    float64 refinement sweeps of a set of mixed decoders whose systems were staged by
     :func:`stage_mixed` (each with at least K intervals).  ``launch`` only
     enqueues device work (capturable in a CUDA graph); ``check`` reads every
     system's flags and correction ratios in one synchronising copy and
@@ -197,29 +190,33 @@ class MixedSolvePlan(object):
         by_K = defaultdict(list)
         for i, d in enumerate(self.decs):
             by_K[d.K].append(i)
-        self.groups = []
-        l = lib()
-        dinv_of = {}
-        for K, idx in sorted(by_K.items()):
-            B = len(idx)
-            nf = int(l.vtb_sym_dinv_floats(K))
-            g = {
-                "K": K, "idx": idx, "ld": self.decs[idx[0]].ld32,
-                "mptrs": torch.as_tensor([self.decs[i].Mr32.data_ptr() for i in idx], dtype=torch.int64, device=dev),
-                "dinv": torch.empty((B, nf), dtype=torch.float32, device=dev),
-                "infos": torch.zeros(B, dtype=torch.int32, device=dev),
-                "flags": torch.zeros(B, dtype=torch.int32, device=dev),
-                "piv": torch.zeros(2 * B, dtype=torch.float64, device=dev),
-            }
-            for j, i in enumerate(idx):
-                dinv_of[i] = g["dinv"][j]
-            self.groups.append(g)
-        self.Kmax = max(d.K for d in self.decs)
-        self.desc_x = trsv_descs([(d.Mr32.data_ptr(), dinv_of[i].data_ptr(), d.xr.data_ptr(), d.ld32, d.K)
-                                  for i, d in enumerate(self.decs)], dev)
-        self.desc_r = trsv_descs([(d.Mr32.data_ptr(), dinv_of[i].data_ptr(), d.rr.data_ptr(), d.ld32, d.K)
-                                  for i, d in enumerate(self.decs)], dev)
-        self.order = [i for g in self.groups for i in g["idx"]]
+        self.groups = [{"K": K, "idx": idx} for K, idx in sorted(by_K.items())]
+        n = len(self.decs)
+        self.flags = torch.zeros(n, dtype=torch.int32, device=dev)
+        self.piv = torch.zeros(2 * n, dtype=torch.float64, device=dev)
+        u64 = lambda xs: np.array(list(xs), np.uint64)
+        Ks = np.array([d.K for d in self.decs], np.int32)
+        nb = np.zeros(1, np.int64)
+        call("vtb_chol_batch_work_bytes", n, Ks.ctypes.data, nb.ctypes.data)
+        self._work = torch.empty(int(nb[0]), dtype=torch.uint8, device=dev)
+        host = np.zeros(int(lib().vtb_chol_batch_bytes(n)), np.uint8)
+        grid = np.zeros(1, np.int32)
+        inverse = [d.inverse_buffers() for d in self.decs]
+        args = [u64(d.Mr32.data_ptr() for d in self.decs), np.array([d.ld32 for d in self.decs], np.int64), Ks,
+                u64(d._cdinv.data_ptr() for d in self.decs), u64(x.data_ptr() for x, _ in inverse),
+                u64(self.flags.data_ptr() + 4 * i for i in range(n)), u64(self.piv.data_ptr() + 16 * i for i in range(n)),
+                np.array([p.rcond * fast.CHOL_MARGIN for p in self.probs], np.float64)]
+        a = [x.ctypes.data for x in args]
+        call("vtb_chol_batch_build", host.ctypes.data, n, a[0], a[1], a[2], a[3], a[4], self._work.data_ptr(), a[5], a[6],
+             a[7], grid.ctypes.data)
+        self._grid = int(grid[0])
+        self._desc = torch.as_tensor(host).to(dev)
+        tiles = np.array([(K + 63) // 64 * ((K + 63) // 64 + 1) // 2 for K in Ks], np.int64)
+        self._tiles = int(tiles.sum())
+        sysd = np.zeros(n, INV_SYSTEM)
+        for i, (d, (linv, work)) in enumerate(zip(self.decs, inverse)):
+            sysd[i] = (linv.data_ptr(), work.data_ptr(), (d.xr.data_ptr(), d.rr.data_ptr()), 0, d.K, tiles[:i].sum())
+        self._systems = torch.as_tensor(np.frombuffer(sysd.tobytes(), np.uint8).copy()).to(dev)
 
     def _fork(self):
         main = torch.cuda.current_stream(self.device)
@@ -237,19 +234,17 @@ class MixedSolvePlan(object):
 
     def launch(self):
         s = stream_ptr()
-        for g in self.groups:
-            rc = self.probs[g["idx"][0]].rcond * fast.CHOL_MARGIN
-            call("vtb_sym_factor_batched", g["mptrs"].data_ptr(), g["ld"], g["K"], len(g["idx"]), rc,
-                 dptr(g["dinv"]), dptr(g["infos"]), dptr(g["flags"]), dptr(g["piv"]), s)
         n = len(self.decs)
-        call("vtb_sym_potrs_batched", dptr(self.desc_x), n, self.Kmax, s)
+        self.flags.zero_()
+        call("vtb_chol_batch_factor", dptr(self._desc), n, self._grid, dptr(self._work), self._work.numel(), s)
+        call("vtb_chol_batch_solve", dptr(self._systems), n, self._tiles, 0, s)
         for i in range(self.sweeps):
             main = self._fork()
             for c, (d, p) in enumerate(zip(self.decs, self.probs)):
                 with torch.cuda.stream(self.streams[c % len(self.streams)]):
                     sweep_residual(d, p, stream_ptr())
             self._join(main)
-            call("vtb_sym_potrs_batched", dptr(self.desc_r), n, self.Kmax, stream_ptr())
+            call("vtb_chol_batch_solve", dptr(self._systems), n, self._tiles, 1, stream_ptr())
             main = self._fork()
             for c, d in enumerate(self.decs):
                 with torch.cuda.stream(self.streams[c % len(self.streams)]):
@@ -263,10 +258,7 @@ class MixedSolvePlan(object):
         """Device tensors (flags, pivots, per-system status words) for
         :meth:`evaluate`; copying them to the host is the caller's choice
         (synchronous in :meth:`check`, asynchronous in the serving loop)."""
-        flags = torch.cat([g["flags"] for g in self.groups])
-        piv = torch.cat([g["piv"] for g in self.groups])
-        stats = torch.stack([d.stat for d in self.decs])
-        return flags, piv, stats
+        return self.flags, self.piv, torch.stack([d.stat for d in self.decs])
 
     def evaluate(self, flags, piv, stats):
         """Indices of the systems the float64 path must decode, from host
@@ -274,15 +266,13 @@ class MixedSolvePlan(object):
         ratios on each decoder."""
         flags, piv, stats = (np.asarray(x) for x in (flags, piv, stats))
         bad = []
-        fl = dict(zip(self.order, flags))
-        pv = {i: (float(piv[2 * j]), float(piv[2 * j + 1])) for j, i in enumerate(self.order)}
         for i, d in enumerate(self.decs):
             tc_err = int(stats[i].view(np.int32)[14])
             if tc_err != 0:
                 raise fast.VtbError("vtb_tc_gemm_bf16", tc_err)
-            d.last_pivots = pv[i]
+            d.last_pivots = (float(piv[2 * i]), float(piv[2 * i + 1]))
             d.last_ratios = [float(x) for x in stats[i][3:3 + min(self.sweeps, 4)]]
-            if fl[i] != 0 or not d._mixed_converged(d.last_ratios):
+            if flags[i] != 0 or not d._mixed_converged(d.last_ratios):
                 bad.append(i)
             else:
                 d.last_solver = "mixed-batched"

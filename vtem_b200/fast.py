@@ -155,9 +155,17 @@ class CoeffDecoder(object):
         self._cdinv = torch.empty(int(lib().vtb_chol_dinv_floats(self.K)), dtype=torch.float32, device=device)
         self._cwork = torch.empty(int(lib().vtb_chol_work_bytes(self.K)), dtype=torch.uint8, device=device)
         if self.mixed_factor == "inverse":
-            self._clinv = torch.empty(int(lib().vtb_chol_inverse_floats(self.K)), dtype=torch.float32, device=device)
+            self.inverse_buffers()
+
+    def inverse_buffers(self):
+        """Device buffers of the tile Cholesky's inverse (its packed tiles,
+        the product solves' scratch) of a mixed decoder."""
+        if getattr(self, "_clinv", None) is None:
+            dev = self.M.device
+            self._clinv = torch.empty(int(lib().vtb_chol_inverse_floats(self.K)), dtype=torch.float32, device=dev)
             # product-solve scratch: partial sums and tickets (zeroed once; every solve leaves it zeroed)
-            self._cy = torch.zeros(int(lib().vtb_chol_solve_inverse_bytes(self.K)), dtype=torch.uint8, device=device)
+            self._cy = torch.zeros(int(lib().vtb_chol_solve_inverse_bytes(self.K)), dtype=torch.uint8, device=dev)
+        return self._clinv, self._cy
 
     def set_norm(self, h_norm):
         """Per-neuron weights norm (vtem/vtdm.py:634-638, 1/(kappa sigma) for
