@@ -218,6 +218,17 @@ int vtb_solve_eq_sym_workspace(int n, int64_t* bytes);
 int vtb_solve_eq_sym(double* G, int64_t ld, const double* q, double* c, int n, double rcond, void* work,
                      int64_t work_bytes, int32_t* kept, void* stream);
 
+/* The same solve for a positive semidefinite G of rank at most about n/2 whose
+ * eigenvalues all lie clear of the truncation (above rcond * max, or rounding
+ * noise): c = G^+ q by a pivoted Cholesky G = L L^T and the r x r system
+ * L^T L, without an eigendecomposition.  *accepted (host) is 1 when that was
+ * certified; else 0, and the caller solves with vtb_solve_eq_sym: G (its lower
+ * triangle is read) is not written either way.  *kept (device, may be NULL)
+ * receives r.  Synchronises the stream. */
+int vtb_solve_psd_workspace(int n, int64_t* bytes);
+int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* c, int n, double rcond, void* work,
+                  int64_t work_bytes, int32_t* kept, int32_t* accepted, void* stream);
+
 /* RNN decoder: c = 0, then steps+1 updates c += dt_alpha (q - G c).  y (may
  * be NULL) receives the last residual, c_tmp is an n-double scratch vector,
  * ynorm_trace (may be NULL) the squared residual norm every trace_every

@@ -48,6 +48,8 @@ SIGNATURES = {
     "vtb_compute_G_work": [P, P, P, I, D, I, P, L, D, I, P, L, P, L, P],
     "vtb_solve_eq_sym_workspace": [I, P],
     "vtb_solve_eq_sym": [P, L, P, P, I, D, P, L, P, P],
+    "vtb_solve_psd_workspace": [I, P],
+    "vtb_solve_psd": [P, L, P, P, I, D, P, L, P, P, P],
     "vtb_rnn": [P, L, P, P, P, P, I, D, I, P, I, P],
     "vtb_reconstruct_workspace": [I, I, I, P],
     "vtb_reconstruct": [P, I, I, P, P, P, P, P, I, P, I, I, D, P, P, L, P],

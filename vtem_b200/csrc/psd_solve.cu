@@ -1,0 +1,582 @@
+// Pseudoinverse solve of a positive semidefinite system of low rank.
+//
+// The plain decoder's Gram G (n x n) has the rank of the Dirichlet space, a
+// fraction of n in any window that samples it well, and its eigenvalues below
+// that rank are rounding noise.  solve_eq_sym's eigendecomposition of G
+// (solve.cu) then spends 4/3 n^3 operations, most of them in a chain of n
+// matrix-vector products, to find a null space it drops.  Here instead
+//   G = L L^T,  L n x r,  by Cholesky with pivoting down to rounding noise,
+//   B = L^T L (r x r, the nonzero eigenvalues of G),
+//   G^+ q = L B^-1 B^-1 L^T q,  refined once with q - G c,
+// which is the reference's truncated pseudoinverse exactly when the rule
+// s > rcond * s_0 drops the noise and keeps the rest.  Both are certified:
+// B - rcond * |B|_inf I has a Cholesky factorisation (every eigenvalue of B
+// passes the rule), and the remainder G - L L^T is below it (by its trace, and
+// by its action on a fixed vector, as an indefinite G could hide from its
+// diagonal).  Anything else is left to the
+// eigendecomposition: *accepted = 0, G untouched.
+//
+// Pivots are taken kPcB at a time: candidates are the largest remaining
+// diagonal entries of kPcB strided groups of indices, their columns of the
+// Schur complement come from one product (C = G(:, cand) - L L(cand, :)^T, the
+// float64 GEMM), and a pivoted Cholesky of the candidates' own block accepts
+// those that stay above a hundredth of the largest diagonal (for a
+// semidefinite matrix any order of such pivots is stable: entries of L are
+// bounded by the square root of the diagonal).  So the chain is one of
+// r / kPcB small launches instead of r global searches.  k, the columns so
+// far, lives on the device (accepted counts vary); the product runs over the
+// host's upper bound, the columns beyond k being zero.
+//
+// Measured at n = 1900, r = 261 (the small configuration): 21.0 ms with the
+// eigendecomposition, 1.1 ms here; n = 24000, r = 1921: 6.9 s and 22 ms.  A
+// matrix of full rank is refused after the first steps (by the trace its
+// columns have taken) or at n/2 columns: 0.2 ms lost of 3.3 at n = 300, 0.4 of
+// 28 at n = 2000.
+#include <cusolverDn.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstddef>
+
+#include "common.cuh"
+#include "gemm_f64.cuh"
+
+namespace vtb {
+
+constexpr int kPcB = 32;               // candidates (and at most as many pivots) per step
+constexpr int kPcMaxRank = 3072;       // columns the workspace holds at most
+constexpr double kPcKeep = 0.01;       // accepted pivots, relative to the largest remaining diagonal
+// pivots end here, relative to G's largest diagonal entry: the noise left by
+// the updates measured up to 1.4e-14 (n = 2000, r = 800)
+constexpr double kPcTol = 1024 * 2.220446049250313e-16;
+
+struct PcState {
+    int k, nacc, done, bad;            // columns; accepted in this step; 1 finished, 2 out of columns; indefinite
+    int cand[kPcB], order[kPcB];       // candidate rows (-1: none); accepted candidates in pivot order
+    double maxd0, tol, dmax;           // largest diagonal entry of G; stop below; largest remaining
+    double trace0;                     // of G
+    double R[kPcB * kPcB];             // factor of the accepted block, row-major lower
+    double trace;                      // of the remainder G - L L^T
+    double probe, norm;                // |G v - L L^T v|_2; |B|_inf
+    int info[2];
+};
+
+__device__ __forceinline__ double warp_max(double v) {
+    for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// d = diag(G), the tolerance, zero state (one block)
+__global__ void __launch_bounds__(1024) pc_init_kernel(const double* __restrict__ G, int64_t ld, int n,
+                                                       double* __restrict__ d, PcState* __restrict__ st) {
+    __shared__ double sm[32], ts[32];
+    double m = 0.0, tr = 0.0;
+    bool neg = false;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double v = G[(int64_t)i * ld + i];
+        d[i] = v;
+        m = fmax(m, v);
+        tr += v;
+        neg |= !(v >= 0.0);
+    }
+    m = warp_max(m);
+    for (int o = 16; o; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    if ((threadIdx.x & 31) == 0) {
+        sm[threadIdx.x >> 5] = m;
+        ts[threadIdx.x >> 5] = tr;
+    }
+    const int any = __syncthreads_or(neg);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) {
+            m = fmax(m, sm[w]);
+            tr += ts[w];
+        }
+        st->trace0 = tr;
+        st->k = st->nacc = st->done = 0;
+        st->bad = any || !(m > 0.0) || !(m < 1e300);
+        st->maxd0 = m;
+        st->tol = kPcTol * m;
+        st->dmax = m;
+        st->probe = st->norm = 0.0;
+        st->info[0] = st->info[1] = 0;
+    }
+}
+
+// the columns accepted last join k; candidates of the next step and their rows of L (32 warps, warp = group)
+__global__ void __launch_bounds__(1024) pc_select_kernel(double* __restrict__ d, int n, const double* __restrict__ L,
+                                                         int64_t ldl, int cols, int used, double* __restrict__ LP,
+                                                         PcState* __restrict__ st) {
+    __shared__ double smax[32], smin[32], ssum[32];
+    __shared__ int s_done;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double best = -1.0, low = 0.0, sum = 0.0;
+    int at = -1;
+    for (int i = w + 32 * lane; i < n; i += 1024) {
+        const double v = d[i];
+        sum += v;
+        low = fmin(low, v);
+        if (v > best) {
+            best = v;
+            at = i;
+        }
+    }
+    for (int o = 16; o; o >>= 1) {
+        const double b2 = __shfl_xor_sync(0xffffffffu, best, o), l2 = __shfl_xor_sync(0xffffffffu, low, o);
+        const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+        low = fmin(low, l2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (b2 > best || (b2 == best && a2 >= 0 && (at < 0 || a2 < at))) {
+            best = b2;
+            at = a2;
+        }
+    }
+    if (lane == 0) {
+        smax[w] = best;
+        smin[w] = low;
+        ssum[w] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double m = smax[0], l = smin[0];
+        for (int k = 1; k < 32; ++k) {
+            m = fmax(m, smax[k]);
+            l = fmin(l, smin[k]);
+            sum += ssum[k];
+        }
+        const int k = st->k + st->nacc;
+        st->k = k;
+        st->nacc = 0;
+        st->dmax = m;
+        if (l < -16.0 * st->tol) st->bad = 1;
+        if (!st->done) {
+            if (!(m > st->tol)) st->done = 1;
+            else if (k + kPcB > cols) st->done = 2;
+            // columns taken largest first reduce the trace less and less, so the
+            // rank is at least k over the share of the trace they have taken
+            else if (k > 0 && (double)k * st->trace0 > 0.55 * n * (st->trace0 - sum)) st->done = 2;
+        }
+        s_done = st->done || st->bad;
+        smax[0] = m;
+    }
+    __syncthreads();
+    const bool use = !s_done && at >= 0 && best > st->tol && best >= kPcKeep * smax[0];
+    if (lane == 0) st->cand[w] = use ? at : -1;
+    for (int j = lane; j < used; j += 32) LP[(int64_t)w * ldl + j] = use ? L[(int64_t)at * ldl + j] : 0.0;
+}
+
+// C[i][j] = G(i, cand_j), from G's lower triangle
+__global__ void __launch_bounds__(256) pc_gather_kernel(const double* __restrict__ G, int64_t ld, int n,
+                                                        double* __restrict__ C, const PcState* __restrict__ st) {
+    const int j = threadIdx.x & 31;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const int c = st->cand[j];
+    C[(int64_t)i * kPcB + j] = c < 0 ? 0.0 : __ldg(G + (int64_t)max(i, c) * ld + min(i, c));
+}
+
+// Pivoted Cholesky of the candidates' block (one warp, lane = candidate): the
+// column of each pivot is formed when it is taken, from the lane's own entries
+// of L (registers) and the pivot's (shared memory), and pivots are ranked by
+// one integer reduction (the diagonal entry's float bits above the lane's
+// number; their exact order does not matter).
+__global__ void __launch_bounds__(32) pc_factor_kernel(const double* __restrict__ C, PcState* __restrict__ st) {
+    __shared__ double S[kPcB][kPcB + 1], Lc[kPcB][kPcB + 1];   // the block; Lc[j][row]
+    const int r = threadIdx.x;
+    const int mine = st->cand[r];
+    const double floor_ = fmax(st->tol, kPcKeep * st->dmax);
+    double rows[kPcB];
+#pragma unroll
+    for (int c = 0; c < kPcB; ++c) {
+        const int row = __shfl_sync(0xffffffffu, mine, c);
+        rows[c] = row >= 0 && mine >= 0 ? C[(int64_t)row * kPcB + r] : 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < kPcB; ++c) S[c][r] = rows[c];
+    __syncwarp();
+    bool left = mine >= 0;
+    double diag = S[r][r];
+    double l[kPcB];
+    int a = 0, at = -1;                                      // at: this lane's place in the pivot order
+#pragma unroll
+    for (int j = 0; j < kPcB; ++j) {
+        l[j] = 0.0;
+        if (a == j) {
+            const unsigned key = left && diag >= floor_ ? (__float_as_uint((float)diag) & ~31u) | (unsigned)r : 0u;
+            const unsigned best = __reduce_max_sync(0xffffffffu, key);
+            if (best >= 32u) {
+                const int p = best & 31u;
+                const double inv = 1.0 / sqrt(__shfl_sync(0xffffffffu, diag, p));
+                double v0 = S[p][r], v1 = 0.0;
+#pragma unroll
+                for (int t = 0; t < j; t += 2) {
+                    v0 = fma(-l[t], Lc[t][p], v0);
+                    if (t + 1 < j) v1 = fma(-l[t + 1], Lc[t + 1][p], v1);
+                }
+                l[j] = r == p ? diag * inv : left ? (v0 + v1) * inv : 0.0;
+                if (r == p) {
+                    left = false;
+                    at = j;
+                }
+                diag = fma(-l[j], l[j], diag);
+                Lc[j][r] = l[j];
+                if (r == 0) st->order[j] = p;
+                a = j + 1;
+                __syncwarp();
+            }
+        }
+    }
+    // R[t][j]: entry of pivot t in column j
+    if (at >= 0) {
+#pragma unroll
+        for (int j = 0; j < kPcB; ++j)
+            if (j <= at) st->R[at * kPcB + j] = l[j];
+    }
+    if (r == 0) st->nacc = a;
+}
+
+// the accepted columns of L: every row of C substituted through R; d less their
+// squares.  Thread = row; rows enter and leave through shared memory, so that
+// global memory sees whole rows of 256 bytes.
+__global__ void __launch_bounds__(64) pc_update_kernel(const double* __restrict__ C, int n, double* __restrict__ L,
+                                                       int64_t ldl, double* __restrict__ d,
+                                                       const PcState* __restrict__ st) {
+    __shared__ double R[kPcB][kPcB];
+    __shared__ double tile[2][32][kPcB + 1];
+    __shared__ double inv[kPcB];
+    __shared__ int ord[kPcB], piv[kPcB];
+    const int a = st->nacc, k = st->k;
+    if (a == 0) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = blockIdx.x * 64 + 32 * w, i = i0 + lane;
+    for (int e = threadIdx.x; e < kPcB * kPcB; e += 64) {
+        const int t = e / kPcB, j = e % kPcB;
+        R[t][j] = t < a && j <= t ? st->R[e] : 0.0;
+    }
+    if (threadIdx.x < kPcB) {
+        const int t = threadIdx.x;
+        inv[t] = t < a ? 1.0 / st->R[t * kPcB + t] : 0.0;
+        ord[t] = t < a ? st->order[t] : 0;
+        piv[t] = t < a ? st->cand[st->order[t]] : -1;
+    }
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) tile[w][r][lane] = i0 + r < n ? C[(int64_t)(i0 + r) * kPcB + lane] : 0.0;
+    __syncthreads();
+    double x[kPcB];
+#pragma unroll
+    for (int t = 0; t < kPcB; ++t) x[t] = t < a ? tile[w][lane][ord[t]] : 0.0;
+    int own = kPcB;                        // row i is the own-th pivot: its later entries are zero by construction
+#pragma unroll
+    for (int t = 0; t < kPcB; ++t)
+        if (piv[t] == i) own = t;
+    double s = 0.0;
+#pragma unroll
+    for (int t = 0; t < kPcB; ++t) {
+        if (t > own) x[t] = 0.0;
+        x[t] *= inv[t];
+        s = fma(x[t], x[t], s);
+#pragma unroll
+        for (int j = t + 1; j < kPcB; ++j) x[j] = fma(-R[j][t], x[t], x[j]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < kPcB; ++t) tile[w][lane][t] = x[t];
+    __syncwarp();
+    if (lane < a)
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r)
+            if (i0 + r < n) L[(int64_t)(i0 + r) * ldl + k + lane] = tile[w][r][lane];
+    if (i < n) d[i] = own < kPcB ? 0.0 : d[i] - s;
+}
+
+// y_b = A^T x_b (row-major A, n x r) for one or two vectors: block of 32 columns x 32 row groups
+__global__ void __launch_bounds__(1024) pc_gemv_t_kernel(const double* __restrict__ A, int64_t ld, int n, int r,
+                                                        const double* __restrict__ x, double* __restrict__ y) {
+    __shared__ double part[32][33];
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+    const double* xv = x + (int64_t)blockIdx.y * n;
+    double s0 = 0.0, s1 = 0.0;
+    if (c < r) {
+        int i = g;
+        for (; i + 32 < n; i += 64) {
+            s0 = fma(A[(int64_t)i * ld + c], xv[i], s0);
+            s1 = fma(A[(int64_t)(i + 32) * ld + c], xv[i + 32], s1);
+        }
+        if (i < n) s0 = fma(A[(int64_t)i * ld + c], xv[i], s0);
+    }
+    part[g][threadIdx.x & 31] = s0 + s1;
+    __syncthreads();
+    if (g == 0 && c < r) {
+        double t = 0.0;
+        for (int k = 0; k < 32; ++k) t += part[k][threadIdx.x & 31];
+        y[(int64_t)blockIdx.y * r + c] = t;
+    }
+}
+
+// y_b = A x_b (+ y_b when add), one warp a row
+__global__ void __launch_bounds__(256) pc_gemv_kernel(const double* __restrict__ A, int64_t ld, int n, int r,
+                                                      const double* __restrict__ x, double* __restrict__ y, int add) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const double* xv = x + (int64_t)blockIdx.y * r;
+    double s = 0.0;
+    for (int j = lane; j < r; j += 32) s = fma(A[(int64_t)i * ld + j], xv[j], s);
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    double* q = y + (int64_t)blockIdx.y * n + i;
+    if (lane == 0) *q = add ? *q + s : s;
+}
+
+// y_b = G x_b from G's lower triangle, b = 0, 1: the part left of the diagonal
+// by rows (one warp each) into y, then the part below it by columns added
+__global__ void __launch_bounds__(256) pc_symv_rows_kernel(const double* __restrict__ G, int64_t ld, int n,
+                                                           const double* __restrict__ x, double* __restrict__ y) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const double* row = G + (int64_t)i * ld;
+    double s = 0.0, t = 0.0;
+    for (int j = lane; j <= i; j += 32) {
+        const double g = row[j];
+        s = fma(g, x[j], s);
+        t = fma(g, x[n + j], t);
+    }
+    for (int o = 16; o; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if (lane == 0) {
+        y[i] = s;
+        y[n + i] = t;
+    }
+}
+
+__global__ void __launch_bounds__(512) pc_symv_cols_kernel(const double* __restrict__ G, int64_t ld, int n,
+                                                           const double* __restrict__ x, double* __restrict__ y) {
+    __shared__ double ps[16][33], pt[16][33];
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+    double s = 0.0, t = 0.0;
+    if (c < n)
+        for (int i = blockIdx.x * 32 + g; i < n; i += 16)
+            if (i > c) {
+                const double v = G[(int64_t)i * ld + c];
+                s = fma(v, x[i], s);
+                t = fma(v, x[n + i], t);
+            }
+    ps[g][threadIdx.x & 31] = s;
+    pt[g][threadIdx.x & 31] = t;
+    __syncthreads();
+    if (g == 0 && c < n) {
+        for (int k = 1; k < 16; ++k) {
+            s += ps[k][threadIdx.x & 31];
+            t += pt[k][threadIdx.x & 31];
+        }
+        y[c] += s;
+        y[n + c] += t;
+    }
+}
+
+// the probe vector: signs by a fixed integer hash
+__global__ void pc_signs_kernel(double* __restrict__ v, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) v[i] = __popc((unsigned)i * 2654435761u ^ ((unsigned)i >> 7)) & 1 ? 1.0 : -1.0;
+}
+
+// res = q - y
+__global__ void pc_residual_kernel(const double* __restrict__ q, const double* __restrict__ y, double* __restrict__ res,
+                                   int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) res[i] = q[i] - y[i];
+}
+
+// st->probe = |y - z|_2, st->trace = sum of |d| (one block)
+__global__ void __launch_bounds__(1024) pc_probe_kernel(const double* __restrict__ y, const double* __restrict__ z,
+                                                        const double* __restrict__ d, int n, PcState* __restrict__ st) {
+    __shared__ double sm[32], tm[32];
+    double s = 0.0, t = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        s = fma(y[i] - z[i], y[i] - z[i], s);
+        t += fabs(d[i]);
+    }
+    for (int o = 16; o; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sm[threadIdx.x >> 5] = s;
+        tm[threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) {
+            s += sm[w];
+            t += tm[w];
+        }
+        st->probe = sqrt(s);
+        st->trace = t;
+    }
+}
+
+// |B|_inf by rows into the state (a maximum of non-negative doubles orders like their bits)
+__global__ void __launch_bounds__(256) pc_norm_kernel(const double* __restrict__ B, int r, PcState* __restrict__ st) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= r) return;
+    double s = 0.0;
+    for (int j = lane; j < r; j += 32) s += fabs(B[(int64_t)i * r + j]);
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(&st->norm), (unsigned long long)__double_as_longlong(s));
+}
+
+__global__ void pc_shift_kernel(const double* __restrict__ B, int r, double rcond, const PcState* __restrict__ st,
+                                double* __restrict__ B2) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= (int64_t)r * r) return;
+    B2[e] = B[e] - (e / r == e % r ? rcond * st->norm : 0.0);
+}
+
+static cusolverDnHandle_t psd_handle(int dev) {
+    static thread_local cusolverDnHandle_t h[64] = {nullptr};
+    if (dev < 0 || dev >= 64) return nullptr;
+    if (!h[dev] && cusolverDnCreate(&h[dev]) != CUSOLVER_STATUS_SUCCESS) h[dev] = nullptr;
+    return h[dev];
+}
+
+struct PsdWork {
+    PcState* st;
+    double *d, *L, *LP, *C, *B, *B2, *v, *y, *t, *wk;
+    int64_t ldl, bytes;
+    int cols;
+};
+
+// columns the factor may take: half of n (beyond it the eigendecomposition is
+// the better one), at most kPcMaxRank, and kPcB of slack
+static int psd_cols(int n) { return (std::min(n / 2, kPcMaxRank) + 2 * kPcB - 1) / kPcB * kPcB; }
+
+static PsdWork psd_work(int n, int lwork, char* base) {
+    PsdWork w;
+    int64_t off = 0;
+    auto take = [&](int64_t doubles) {
+        char* p = base + off;
+        off += (doubles * 8 + 255) & ~(int64_t)255;
+        return reinterpret_cast<double*>(p);
+    };
+    w.cols = psd_cols(n);
+    w.ldl = w.cols;
+    w.st = reinterpret_cast<PcState*>(take((sizeof(PcState) + 7) / 8));
+    w.d = take(n);
+    w.L = take((int64_t)n * w.ldl);
+    w.LP = take((int64_t)kPcB * w.ldl);
+    w.C = take((int64_t)n * kPcB);
+    w.B = take((int64_t)w.cols * w.cols);
+    w.B2 = take((int64_t)w.cols * w.cols);
+    w.v = take(2 * (int64_t)n);
+    w.y = take(2 * (int64_t)n);
+    w.t = take(2 * (int64_t)w.cols);
+    w.wk = take(lwork);
+    w.bytes = off;
+    return w;
+}
+
+static int psd_lwork(cusolverDnHandle_t h, int n, int* lwork) {
+    return cusolverDnDpotrf_bufferSize(h, CUBLAS_FILL_MODE_LOWER, psd_cols(n), nullptr, psd_cols(n), lwork) ==
+                   CUSOLVER_STATUS_SUCCESS ? VTB_OK : VTB_CUDA_ERR;
+}
+
+}  // namespace vtb
+
+using namespace vtb;
+
+VTB_API int vtb_solve_psd_workspace(int n, int64_t* bytes) {
+    VTB_CHECK_ARG(n > 0 && bytes);
+    int dev = 0, lwork = 0;
+    VTB_CUDA_TRY(cudaGetDevice(&dev));
+    cusolverDnHandle_t h = psd_handle(dev);
+    if (!h) return VTB_CUDA_ERR;
+    const int st = psd_lwork(h, n, &lwork);
+    if (st) return st;
+    *bytes = psd_work(n, lwork, nullptr).bytes;
+    return VTB_OK;
+}
+
+VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* c, int n, double rcond, void* work,
+                          int64_t work_bytes, int32_t* kept, int32_t* accepted, void* stream) {
+    VTB_CHECK_ARG(n > 0 && ld >= n && G && q && c && work && accepted && ((uintptr_t)work & 255) == 0);
+    *accepted = 0;
+    if (!(rcond >= 100.0 * kPcTol) || !(rcond < 1.0)) return VTB_OK;   // the rule would keep noise
+    int dev = 0, lwork = 0;
+    VTB_CUDA_TRY(cudaGetDevice(&dev));
+    cusolverDnHandle_t h = psd_handle(dev);
+    if (!h) return VTB_CUDA_ERR;
+    int st = psd_lwork(h, n, &lwork);
+    if (st) return st;
+    const PsdWork w = psd_work(n, lwork, reinterpret_cast<char*>(work));
+    VTB_CHECK_ARG(work_bytes >= w.bytes);
+    cudaStream_t s = as_stream(stream);
+    if (cusolverDnSetStream(h, s) != CUSOLVER_STATUS_SUCCESS) return VTB_CUDA_ERR;
+    VTB_CUDA_TRY(cudaMemsetAsync(w.L, 0, (size_t)n * w.ldl * 8, s));
+    pc_init_kernel<<<1, 1024, 0, s>>>(G, ld, n, w.d, w.st);
+    struct {
+        int k, nacc, done, bad;
+    } host = {0, 0, 0, 0};
+    constexpr int kCheck = 4;              // steps between looks at the state
+    const int most = 2 * (w.cols / kPcB) + kCheck;
+    for (int step = 0; step < most && !host.done && !host.bad; ++step) {
+        const int cols = std::min(step * kPcB, w.cols);      // k is at most this
+        pc_select_kernel<<<1, 1024, 0, s>>>(w.d, n, w.L, w.ldl, w.cols, cols, w.LP, w.st);
+        pc_gather_kernel<<<ceil_div(n, 8), 256, 0, s>>>(G, ld, n, w.C, w.st);
+        if (cols) {
+            const GemmF64Args g{n, kPcB, cols, w.L, w.ldl, 1, w.LP, w.ldl, 1, w.C, kPcB, 1, -1.0, 1.0};
+            st = gemm_f64(g, s);
+            if (st) return st;
+        }
+        pc_factor_kernel<<<1, 32, 0, s>>>(w.C, w.st);
+        pc_update_kernel<<<ceil_div(n, 64), 64, 0, s>>>(w.C, n, w.L, w.ldl, w.d, w.st);
+        if (step % kCheck == kCheck - 1 || step + 1 == most) {
+            VTB_CUDA_TRY(cudaMemcpyAsync(&host, w.st, sizeof(host), cudaMemcpyDeviceToHost, s));
+            VTB_CUDA_TRY(cudaStreamSynchronize(s));
+        }
+    }
+    st = launch_status();
+    if (st) return st;
+    if (host.done != 1 || host.bad || host.k < 1) return VTB_OK;
+    const int r = host.k;
+    const GemmF64Args gb{r, r, n, w.L, 1, w.ldl, w.L, 1, w.ldl, w.B, r, 1, 1.0, 0.0};
+    st = gemm_f64(gb, s);
+    if (st) return st;
+    pc_norm_kernel<<<ceil_div((int64_t)r * 32, 256), 256, 0, s>>>(w.B, r, w.st);
+    pc_shift_kernel<<<ceil_div((int64_t)r * r, 256), 256, 0, s>>>(w.B, r, rcond, w.st, w.B2);
+    int* info = reinterpret_cast<int*>(reinterpret_cast<char*>(w.st) + offsetof(PcState, info));
+    if (cusolverDnDpotrf(h, CUBLAS_FILL_MODE_LOWER, r, w.B2, r, w.wk, lwork, info + 1) != CUSOLVER_STATUS_SUCCESS ||
+        cusolverDnDpotrf(h, CUBLAS_FILL_MODE_LOWER, r, w.B, r, w.wk, lwork, info) != CUSOLVER_STATUS_SUCCESS)
+        return VTB_CUDA_ERR;
+    int* unused = reinterpret_cast<int*>(w.wk);
+    // c (+)= L B^-1 B^-1 L^T x
+    auto apply = [&](const double* x, int add) -> int {
+        pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, x, w.t);
+        for (int i = 0; i < 2; ++i)
+            if (cusolverDnDpotrs(h, CUBLAS_FILL_MODE_LOWER, r, 1, w.B, r, w.t, r, unused) != CUSOLVER_STATUS_SUCCESS)
+                return VTB_CUDA_ERR;
+        pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, c, add);
+        return VTB_OK;
+    };
+    if ((st = apply(q, 0))) return st;
+    // one pass over G for the refinement (x = c) and the probe (x = signs)
+    VTB_CUDA_TRY(cudaMemcpyAsync(w.v, c, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
+    pc_signs_kernel<<<ceil_div(n, 256), 256, 0, s>>>(w.v + n, n);
+    pc_symv_rows_kernel<<<ceil_div((int64_t)n * 32, 256), 256, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_symv_cols_kernel<<<ceil_div(n, 32), 512, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, w.v + n, w.t);
+    pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, w.v + n, 0);
+    pc_probe_kernel<<<1, 1024, 0, s>>>(w.y + n, w.v + n, w.d, n, w.st);
+    pc_residual_kernel<<<ceil_div(n, 256), 256, 0, s>>>(q, w.y, w.v, n);
+    if ((st = apply(w.v, 1))) return st;
+    PcState end;
+    VTB_CUDA_TRY(cudaMemcpyAsync(&end, w.st, sizeof(end), cudaMemcpyDeviceToHost, s));
+    if (kept) VTB_CUDA_TRY(cudaMemcpyAsync(kept, w.st, 4, cudaMemcpyDeviceToDevice, s));
+    VTB_CUDA_TRY(cudaStreamSynchronize(s));
+    st = launch_status();
+    if (st) return st;
+    // the remainder against the rule, with s_0 at least the largest diagonal entry and |B|_inf / sqrt(r)
+    const double rule = rcond * std::max(end.maxd0, end.norm / std::sqrt((double)r));
+    if (end.info[0] != 0 || end.info[1] != 0 || !(end.trace <= 0.1 * rule) || !(end.probe <= 0.05 * rule)) return VTB_OK;
+    *accepted = 1;
+    return VTB_OK;
+}

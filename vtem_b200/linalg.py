@@ -9,12 +9,20 @@ from ._abi import call, dptr, stream_ptr
 
 F64 = torch.float64
 
+# below this size the low-rank solve's steps (0.7 ms at n = 500, against 5.0 for
+# the eigendecomposition) save little and a refusal costs most
+PSD_MIN_SIZE = 256
+
 
 def solve_eq_sym(G, q, rcond=1e-8, return_kept=False):
     """Solve G c = q for symmetric G by pseudoinversion, dropping singular
     values at or below ``rcond * s_0`` (linalg.py:591-631).  As in the
-    reference, G is destroyed (it holds the eigenvectors afterwards).  Only
-    G's lower triangle is read."""
+    reference, G may be destroyed.  Only G's lower triangle is read.
+
+    A positive semidefinite G of low rank (a spike Gram with more intervals
+    than the Dirichlet space has dimensions) is solved through its pivoted
+    Cholesky factor where no eigenvalue lies near the truncation; any other G
+    by its eigendecomposition, in place."""
     if not isinstance(G, torch.Tensor) or not isinstance(q, torch.Tensor):
         raise TypeError("G, q must be CUDA tensors")
     if G.dtype != q.dtype:
@@ -29,6 +37,19 @@ def solve_eq_sym(G, q, rcond=1e-8, return_kept=False):
     if not G.is_contiguous():
         raise ValueError("G must be contiguous")
     nbytes = np.zeros(1, np.int64)
+    if n >= PSD_MIN_SIZE:
+        call("vtb_solve_psd_workspace", n, nbytes.ctypes.data)
+        work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device=G.device)
+        qv = q.reshape(-1).contiguous()
+        c = torch.empty_like(qv)
+        kept = torch.zeros(1, dtype=torch.int32, device=G.device)
+        accepted = np.zeros(1, np.int32)
+        call("vtb_solve_psd", dptr(G), n, dptr(qv), dptr(c), n, float(rcond), dptr(work), int(nbytes[0]), dptr(kept),
+             accepted.ctypes.data, stream_ptr())
+        if accepted[0]:
+            c = c.reshape(q.shape)
+            return (c, int(kept.item())) if return_kept else c
+        del work
     call("vtb_solve_eq_sym_workspace", n, nbytes.ctypes.data)
     work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device=G.device)
     qv = q.reshape(-1).contiguous()
