@@ -166,6 +166,13 @@ int vtb_spike_pairs(const double* spike_time, const int32_t* spike_step, const i
                     int block_frames, double refresh_interval, double t0, double T, const int64_t* offsets,
                     double* tk1, double* tk2, int32_t* ind, int32_t* outside, void* stream);
 
+/* Before vtb_spike_pairs: offsets[n] = the pairs of the neurons before n,
+ * meta[0] = all pairs, meta[1] = 1 if a spike lies outside (t0, t0 + T) (two
+ * int64 in device memory, one host read for both). */
+int vtb_spike_offsets(const double* spike_time, const int32_t* spike_step, const int32_t* spike_count, int N, int cap,
+                      int block_frames, double refresh_interval, double t0, double T, int64_t* offsets, int64_t* meta,
+                      void* stream);
+
 /* ------------------------------------------------------------ Dirichlet space */
 
 /* Dirichlet coefficients Ds (N, 2My+1, 2Mx+1) complex from RFs sampled on

@@ -39,6 +39,7 @@ SIGNATURES = {
     "vtb_gemm_f64": [I, I, I, P, L, L, P, L, L, P, L, L, D, D, P],
     "vtb_iaf_encode": [P, L, L, I, I, I, D, P, P, P, P, P, P, L, L, L, I, P, P, P, P, P, I, P, D, P, D, P],
     "vtb_spike_pairs": [P, P, P, I, I, I, D, D, D, P, P, P, P, P, P],
+    "vtb_spike_offsets": [P, P, P, I, I, I, D, D, D, P, P, P],
     "vtb_dirichlet_coeffs": [P, I, I, I, L, I, I, D, P, P],
     "vtb_dirich_space": [P, I, I, I, I, I, I, I, P, P],
     "vtb_dsw": [P, I, I, P, P, L, P],

@@ -404,6 +404,56 @@ __global__ void __launch_bounds__(kIafWarps * 32, 1) iaf_scan_kernel(const __gri
     }
 }
 
+// offs[n] = pairs of the neurons before n (max(count - 1, 0) each), meta[0] =
+// all of them (one block, any N).  Bound: launches and host reads; with
+// spike_window_kernel it takes the place of five torch launches, and of one of
+// the two reads that the pairs' count and the window test took (encoding and
+// pairing 1024 neurons x 10,000 samples: 418 -> 378 us).
+__global__ void __launch_bounds__(1024) spike_offsets_kernel(const int32_t* __restrict__ count, int N,
+                                                             int64_t* __restrict__ offs, int64_t* __restrict__ meta) {
+    __shared__ int64_t s_w[32];
+    __shared__ int64_t s_base;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_base = 0;
+    __syncthreads();
+    for (int n0 = 0; n0 < N; n0 += 1024) {
+        const int n = n0 + threadIdx.x;
+        const int64_t c = n < N ? max(count[n] - 1, 0) : 0;
+        int64_t x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_w[w] = x;
+        __syncthreads();
+        int64_t before = s_base;
+        for (int k = 0; k < w; ++k) before += s_w[k];
+        if (n < N) offs[n] = before + x - c;
+        __syncthreads();
+        if (threadIdx.x == 1023) s_base = before + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) meta[0] = s_base;
+}
+
+// meta[1] = 1 if a spike lies outside (0, T); one warp per neuron
+__global__ void __launch_bounds__(256) spike_window_kernel(const double* __restrict__ time,
+                                                           const int32_t* __restrict__ step,
+                                                           const int32_t* __restrict__ count, int N, int cap, int bstep,
+                                                           double R, double t0, double T, int64_t* __restrict__ meta) {
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (n >= N) return;
+    const int c = min(count[n], cap);
+    bool bad = false;
+    for (int j = lane; j < c; j += 32) {
+        const int64_t k = (int64_t)n * cap + j;
+        const double t = time[k] + (double)(step[k] / bstep) * R - t0;
+        bad |= !(t > 0.0 && t < T);
+    }
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(reinterpret_cast<unsigned long long*>(meta + 1), 1ull);
+}
+
 // Consecutive pairs of each neuron's spikes, one warp per neuron (this file
 // is compiled without FMA contraction, so t rounds as the reference's
 // expression time + block * refresh - t0 does).
@@ -472,5 +522,19 @@ VTB_API int vtb_spike_pairs(const double* spike_time, const int32_t* spike_step,
     spike_pairs_kernel<<<ceil_div((int64_t)N * 32, 256), 256, 0, as_stream(stream)>>>(
         spike_time, spike_step, spike_count, N, cap, block_frames - 1, refresh_interval, t0, T, offsets, tk1, tk2,
         ind, outside);
+    return launch_status();
+}
+
+VTB_API int vtb_spike_offsets(const double* spike_time, const int32_t* spike_step, const int32_t* spike_count, int N,
+                              int cap, int block_frames, double refresh_interval, double t0, double T, int64_t* offsets,
+                              int64_t* meta, void* stream) {
+    VTB_CHECK_ARG(N >= 0 && cap >= 1 && block_frames >= 2 && meta);
+    cudaStream_t s = as_stream(stream);
+    VTB_CUDA_TRY(cudaMemsetAsync(meta, 0, 16, s));
+    if (N == 0) return VTB_OK;
+    VTB_CHECK_ARG(spike_time && spike_step && spike_count && offsets);
+    spike_offsets_kernel<<<1, 1024, 0, s>>>(spike_count, N, offsets, meta);
+    spike_window_kernel<<<ceil_div((int64_t)N * 32, 256), 256, 0, s>>>(spike_time, spike_step, spike_count, N, cap,
+                                                                      block_frames - 1, refresh_interval, t0, T, meta);
     return launch_status();
 }

@@ -256,17 +256,18 @@ def device_pairs(spikes, T, t0=0.0):
         raise ValueError("device_pairs covers the whole-clip window only")
     N, cap = spikes.time.shape
     dev = spikes.time.device
-    c1 = (spikes.count.long() - 1).clamp_(min=0)
-    incl = torch.cumsum(c1, 0)
-    n = int(incl[-1]) if N else 0
-    offs = incl - c1
+    scratch = torch.empty(N + 2, dtype=torch.int64, device=dev)      # pairs before each neuron, then (all, outside)
+    offs, meta = scratch[:N], scratch[N:]
+    call("vtb_spike_offsets", dptr(spikes.time), dptr(spikes.step), dptr(spikes.count), N, cap, spikes.block_frames,
+         spikes.refresh_interval, float(t0), float(T), dptr(offs) if N else None, dptr(meta), stream_ptr())
+    n, outside = meta.tolist()
+    if outside:
+        raise ValueError("spikes outside the window: use read_select_spikes")
     tk1 = torch.empty(n, dtype=torch.float64, device=dev)
     tk2 = torch.empty(n, dtype=torch.float64, device=dev)
     ind = torch.empty(n, dtype=torch.int32, device=dev)
-    outside = torch.zeros(1, dtype=torch.int32, device=dev)
-    call("vtb_spike_pairs", dptr(spikes.time), dptr(spikes.step), dptr(spikes.count), N, cap, spikes.block_frames,
-         spikes.refresh_interval, float(t0), float(T), dptr(offs), dptr(tk1) if n else None,
-         dptr(tk2) if n else None, dptr(ind) if n else None, dptr(outside), stream_ptr())
-    if int(outside.item()):
-        raise ValueError("spikes outside the window: use read_select_spikes")
+    if n:
+        call("vtb_spike_pairs", dptr(spikes.time), dptr(spikes.step), dptr(spikes.count), N, cap, spikes.block_frames,
+             spikes.refresh_interval, float(t0), float(T), dptr(offs), dptr(tk1), dptr(tk2), dptr(ind), dptr(meta),
+             stream_ptr())
     return tk1, tk2, ind
