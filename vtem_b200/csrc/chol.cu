@@ -261,12 +261,13 @@ __device__ int cta_ready2(const unsigned* f1, unsigned v1, const unsigned* f2, u
 
 // shared tile s into tile (I, J) of A (rows and columns below K; for a
 // diagonal tile the lower triangle only)
-__device__ void store_tile(const CholCtx& c, const float* s, int I, int J) {
+__device__ void store_tile(const CholCtx& c, const float* s, int I, int J, int tid = threadIdx.x,
+                           int nthreads = kCThreads) {
     const int r0 = I * kCT, c0 = J * kCT;
     if (r0 + kCT <= c.K && c0 + kCT <= c.K && (c.ld & 3) == 0 && ((uintptr_t)c.A & 15) == 0) {
         // full tile: 16-byte stores (4 rows of a column); a diagonal tile keeps
         // the matrix's upper triangle (chunks across the diagonal entry by entry)
-        for (int e = threadIdx.x; e < kCTE / 4; e += kCThreads) {
+        for (int e = tid; e < kCTE / 4; e += nthreads) {
             const int cc = e >> 4, r = (e & 15) * 4;
             float* g = c.A + (int64_t)(c0 + cc) * c.ld + r0 + r;
             const float4 v = reinterpret_cast<const float4*>(s)[e];
@@ -280,7 +281,7 @@ __device__ void store_tile(const CholCtx& c, const float* s, int I, int J) {
         }
         return;
     }
-    for (int e = threadIdx.x; e < kCTE; e += kCThreads) {
+    for (int e = tid; e < kCTE; e += nthreads) {
         const int cc = e >> 6, r = e & 63;
         const int gr = r0 + r, gc = c0 + cc;
         if (gr < c.K && gc < c.K && (I != J || r >= cc)) __stcg(c.A + (int64_t)gc * c.ld + gr, s[e]);
@@ -315,17 +316,33 @@ __device__ __forceinline__ void sub_ptq(float (&acc)[4][4], const float* P, cons
     }
 }
 
-// acc[i][j] -= sum_t P[t][4tr+i] Q[4tc+j][t]  (P column-major 64 x 64; Q with the t index contiguous: Q[c][t]
-// at Q + c*64 + t).  The Q reads of a quarter-warp are one address (same tc): broadcasts.
-__device__ __forceinline__ void sub_pq_rowq(float (&acc)[4][4], const float* P, const float* Q, int tr, int tc) {
+// The products with a triangular factor (Q = L^-1 or X_ii, row-major: row c holds
+// t <= c) stop each warp at the last t that its columns reach.  A warp covers
+// the 8 columns of block p; warps w and w + 4 share a scheduler, so they take
+// the blocks p and 7 - p: 72 of the 128 column steps on each.  On one CTA the
+// 64 x 64 x 64 product took 3700 cycles with every t, 256 threads x 4 x 4.
+struct TriMap {
+    int tr, tc, tend;
+    __device__ __forceinline__ TriMap() {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int p = w < 4 ? w : 11 - w;
+        tr = lane & 15;
+        tc = 2 * p + (lane >> 4);
+        tend = 8 * p + 8;
+    }
+};
+
+// acc[i][j] -= sum_{t < tend} P[t][4tr+i] Q[4tc+j][t]  (P column-major 64 x 64; Q with the t index contiguous:
+// Q[c][t] at Q + c*64 + t).  The Q reads of a half-warp are one address (same tc): broadcasts.
+__device__ __forceinline__ void sub_pq_tri(float (&acc)[4][4], const float* P, const float* Q, const TriMap& m) {
 #pragma unroll 2
-    for (int t = 0; t < kCT; t += 4) {
+    for (int t = 0; t < m.tend; t += 4) {
         float4 q[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) q[j] = *reinterpret_cast<const float4*>(Q + (4 * tc + j) * kCT + t);
+        for (int j = 0; j < 4; ++j) q[j] = *reinterpret_cast<const float4*>(Q + (4 * m.tc + j) * kCT + t);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const float4 p = *reinterpret_cast<const float4*>(P + (t + u) * kCT + 4 * tr);
+            const float4 p = *reinterpret_cast<const float4*>(P + (t + u) * kCT + 4 * m.tr);
             float qv[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) qv[j] = u == 0 ? q[j].x : u == 1 ? q[j].y : u == 2 ? q[j].z : q[j].w;
@@ -336,16 +353,20 @@ __device__ __forceinline__ void sub_pq_rowq(float (&acc)[4][4], const float* P, 
 
 __device__ __forceinline__ void acc_from(float (&acc)[4][4], const float* s, int tr, int tc) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = s[(4 * tc + j) * kCT + 4 * tr + i];
+    for (int j = 0; j < 4; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(s + (4 * tc + j) * kCT + 4 * tr);
+        acc[0][j] = v.x;
+        acc[1][j] = v.y;
+        acc[2][j] = v.z;
+        acc[3][j] = v.w;
+    }
 }
 
 __device__ __forceinline__ void acc_to(const float (&acc)[4][4], float* s, int tr, int tc) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[(4 * tc + j) * kCT + 4 * tr + i] = acc[i][j];
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4*>(s + (4 * tc + j) * kCT + 4 * tr) =
+            make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
 }
 
 // ---------------------------------------------------------------- 64 x 64 POTRF
@@ -660,8 +681,9 @@ __device__ __forceinline__ void load_flat(float* s, const float* src) {
 }
 
 // shared 64 x 64 floats to global dst (16-byte aligned)
-__device__ __forceinline__ void store_flat(float* dst, const float* s) {
-    for (int e = threadIdx.x; e < kCTE / 4; e += kCThreads)
+__device__ __forceinline__ void store_flat(float* dst, const float* s, int tid = threadIdx.x,
+                                           int nthreads = kCThreads) {
+    for (int e = tid; e < kCTE / 4; e += nthreads)
         __stcg(reinterpret_cast<float4*>(dst) + e, reinterpret_cast<const float4*>(s)[e]);
 }
 
@@ -763,7 +785,7 @@ __device__ bool task_inverse_final(const CholCtx& c, CholSmem& sm, int i, int j)
         acc_zero(acc);
     }
     if (!inv_accumulate(c, sm, i, j, i - 1, i - 1, acc)) return false;
-    // acc = -S.  With P = -S row-major and Q = X_ii row-major, sub_pq_rowq
+    // acc = -S.  With P = -S row-major and Q = X_ii row-major, sub_pq_tri
     // gives out[a][b] = sum_t S[t][a] X_ii[b][t] = (X_ii S)[b][a]; X_ij = -(X_ii S)
     if (!cta_wait(c, c.xflag + i * T + i, 1u, &sm.ok)) return false;
     load_flat(sm.b[0], c.Xinv + packed_tile(i, i) * kCTE);
@@ -775,10 +797,11 @@ __device__ bool task_inverse_final(const CholCtx& c, CholSmem& sm, int i, int j)
     __syncthreads();
     float out[4][4];
     acc_zero(out);
-    sub_pq_rowq(out, sm.x, sm.b[0], tr, tc);
+    const TriMap m;
+    sub_pq_tri(out, sm.x, sm.b[0], m);
     __syncthreads();
     acc_neg(out);
-    acc_to(out, sm.x, tr, tc);     // X_ij[4tc+q][4tr+p] at (4tc+q)*64 + 4tr+p: row-major
+    acc_to(out, sm.x, m.tr, m.tc);     // X_ij[4tc+q][4tr+p] at (4tc+q)*64 + 4tr+p: row-major
     __syncthreads();
     store_flat(X, sm.x);
     cta_publish(c.xflag + i * T + j, 1u);
@@ -875,10 +898,11 @@ __device__ bool worker_task(const CholCtx& c, CholSmem& sm, int t) {
         __syncthreads();
         float out[4][4];
         acc_zero(out);
-        sub_pq_rowq(out, sm.x, sm.b[0], tr, tc);
+        const TriMap m;
+        sub_pq_tri(out, sm.x, sm.b[0], m);
         __syncthreads();
         acc_neg(out);
-        acc_to(out, sm.x, tr, tc);
+        acc_to(out, sm.x, m.tr, m.tc);
     }
     __syncthreads();
     store_tile(c, sm.x, I, J);
@@ -891,9 +915,9 @@ __device__ bool worker_task(const CholCtx& c, CholSmem& sm, int t) {
 // L_kk^-T, and the next diagonal tile's last update.
 __device__ void diagonal(const CholCtx& c, CholSmem& sm) {
     const int T = c.T;
-    const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool inv = c.Xinv != nullptr;
+    constexpr int kSyrkWarps = 5;        // 136 patches
     float pmin = 3.4e38f, pmax = 0.f;
     int bad = 0;
     int cur = 0;                         // sm.a[cur]: the diagonal tile of this step
@@ -936,11 +960,24 @@ __device__ void diagonal(const CholCtx& c, CholSmem& sm) {
         potrf_inv64(c, D, E, sm.rinv, pmin, pmax, bad, c.K - k * kCT, la, &sm.panel_done);
         // the workers need L_kk^-T first (their TRSMs); L_kk itself and the
         // packed X_kk are written after the sub-diagonal tile is out, so the
-        // release stores on this CTA's path wait for as few stores as possible
+        // release store waits for as few stores as possible
         store_flat(c.Dinv + (int64_t)k * kCTE, E);
-        cta_publish(c.tflag + k * T + k, 2u);
-        // X_{k-1,k-1} was stored during the previous step: this release covers it
-        if (inv && k > 0 && threadIdx.x == 0) c_st_release(c.xflag + (k - 1) * T + k - 1, 1u);
+        // warp 7's last poll (tiles its previous poll saw set); its copies
+        // (every thread's, at step 0) are complete for everyone after the barrier
+        if (threadIdx.x >= kCThreads - 32) {
+            look_ahead_poll(c, la);
+            if (threadIdx.x == kCThreads - 32) sm.la = la.issued;
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        const int pre = sm.la;
+        // warp 0 has the least of the product below: the others do not wait
+        // for its release.  X_{k-1,k-1} was stored during the previous step:
+        // the release covers it.
+        if (threadIdx.x == 0) {
+            c_st_release(c.tflag + k * T + k, 2u);
+            if (inv && k > 0) c_st_release(c.xflag + (k - 1) * T + k - 1, 1u);
+        }
         if (k + 1 >= T) {
             store_tile(c, D, k, k);
             if (inv) {
@@ -949,56 +986,56 @@ __device__ void diagonal(const CholCtx& c, CholSmem& sm) {
             }
             break;
         }
-        // warp 7's last poll (tiles its previous poll saw set), then its
-        // copies are complete for everyone after this barrier
-        if (threadIdx.x >= kCThreads - 32) {
-            look_ahead_poll(c, la);
-            cp_async_wait_all();
-            if (threadIdx.x == kCThreads - 32) sm.la = la.issued;
-        }
-        __syncthreads();
-        const int pre = sm.la;
         // sub-diagonal tile: the workers applied updates k' < k (none when k = 0);
         // L_{k+1,k} = X L_kk^-T
         if (!hx && !(pre & 1)) {
             if (!cta_wait(c, c.tflag + (k + 1) * T + k, 1u, &sm.ok)) return;
             load_tile(c, X, k + 1, k);
+            cp_async_wait_all();
+            __syncthreads();
         }
-        cp_async_wait_all();
-        __syncthreads();
         {
             float out[4][4];
+            const TriMap m;
             acc_zero(out);
-            sub_pq_rowq(out, X, E, tr, tc);
+            sub_pq_tri(out, X, E, m);
             __syncthreads();
             acc_neg(out);
-            acc_to(out, X, tr, tc);
+            acc_to(out, X, m.tr, m.tc);
         }
-        __syncthreads();
-        // L_{k+1,k}, L_kk and the packed X_kk go out now and drain during the
-        // SYRK; L_{k+1,k}'s flag is released after it (the workers need that
-        // tile several microseconds later), by a thread outside warp 0 so
-        // that the next block factorisation does not wait on the release
-        store_tile(c, X, k + 1, k);
-        store_tile(c, D, k, k);
-        if (inv) store_flat(c.Xinv + packed_tile(k, k) * kCTE, E);     // flag set with the next step's release
         // next diagonal tile: the workers applied updates k' < k; this CTA applies k
         if (!hy && !(pre & 2)) {
             if (!cta_wait(c, c.tflag + (k + 1) * T + k + 1, 1u, &sm.ok)) return;
             load_tile(c, Y, k + 1, k + 1);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        // lower 4 x 4 patches only (the factorisation reads the lower triangle)
-        float acc[4][4];
-        if (tc <= tr) {
-            acc_from(acc, Y, tr, tc);
-            sub_ptq(acc, X, X, tr, tc, 0, kCT);
+            cp_async_wait_all();
         }
         __syncthreads();
-        if (tc <= tr) acc_to(acc, Y, tr, tc);
+        // Warps 0-4 update the lower 4 x 4 patches of the next diagonal tile (the
+        // factorisation reads no others; column by column, so that a warp's
+        // rows follow each other) while warps 5-7 write L_{k+1,k}, L_kk and the
+        // packed X_kk (its flag is set with the next step's release) and publish
+        // L_{k+1,k}.  All 256 threads on the update with half of the lanes
+        // masked, after the stores: 4000 + 1700 cycles of the step's 25,800.
+        if (w < kSyrkWarps) {
+            int q = threadIdx.x, pc = 0;
+            while (pc < 16 && q >= 16 - pc) q -= 16 - pc++;
+            if (pc < 16) {
+                const int pr = pc + q;
+                float acc[4][4];
+                acc_from(acc, Y, pr, pc);
+                sub_ptq(acc, X, X, pr, pc, 0, kCT);
+                acc_to(acc, Y, pr, pc);
+            }
+        } else {
+            const int tid = threadIdx.x - 32 * kSyrkWarps;
+            constexpr int n = kCThreads - 32 * kSyrkWarps;
+            store_tile(c, X, k + 1, k, tid, n);
+            asm volatile("bar.sync 2, %0;" ::"n"(n) : "memory");
+            if (tid == 0) c_st_release(c.tflag + (k + 1) * T + k, 2u);
+            store_tile(c, D, k, k, tid, n);
+            if (inv) store_flat(c.Xinv + packed_tile(k, k) * kCTE, E, tid, n);
+        }
         __syncthreads();
-        if (threadIdx.x == kCThreads - 32) c_st_release(c.tflag + (k + 1) * T + k, 2u);
         cur ^= 1;
     }
     // pivot test (pivots of warp 0, which ran every 8 x 8 factorisation)
@@ -1014,7 +1051,7 @@ __device__ void diagonal(const CholCtx& c, CholSmem& sm) {
     }
 }
 
-__global__ void __launch_bounds__(kCThreads, 1) chol_tiles_kernel(CholCtx c) {
+__global__ void __launch_bounds__(kCThreads, 2) chol_tiles_kernel(CholCtx c) {
     extern __shared__ __align__(16) uint8_t chol_smem[];
     CholSmem& sm = *reinterpret_cast<CholSmem*>(chol_smem);
     if (blockIdx.x == 0) diagonal(c, sm);
@@ -1101,7 +1138,10 @@ static int chol_launch(float* A, int64_t ld, int K, float* Dinv, float* Linv, vo
     const bool inv = Linv != nullptr;
     const int ntask = task_count(T, inv);
     const int need = (inv && factor_count(T) > 0 && inverse_count(T) > 0) ? 2 : 1;
-    const int grid = 1 + std::max(need, std::min(nsm - 1, ntask));
+    // two CTAs per SM: a worker's waits and loads run beside the other's products
+    // (factor and inverse, one against two: K = 1017 197 / 197 us, 1921 431 / 392,
+    // 3000 1213 / 953)
+    const int grid = 1 + std::max(need, std::min(std::min(per_sm, 2) * nsm - 1, ntask));
     cudaStream_t s = as_stream(stream);
     const int64_t fbytes = ((int64_t)T * T * 4 + 255) & ~(int64_t)255;
     VTB_CUDA_TRY(cudaMemsetAsync(work, 0, (size_t)(3 * fbytes + 256), s));
