@@ -494,22 +494,45 @@ __global__ void split_bf16x3_kernel(const InT* __restrict__ src, int rows, int K
 }
 
 // dst[r][seg*Kp + k]: seg 0 = hi, seg 1 = lo (the three-product mode's
-// layout).  A thread converts 8 consecutive k and writes 16 bytes per part.
-template <typename InT>
+// layout).  A thread converts 8 consecutive k and writes 16 bytes per part;
+// VEC (k contiguous, every row on 16 bytes) reads them 16 bytes at a time.
+// Bound: memory.  4999 x 2304 float32 (46 MB read, 46 MB written): 15.5 us,
+// against 46 us for a float64 copy and 28 us for its split; with the float32
+// entries converted to float64 and back 20 us.
+template <typename InT, bool VEC>
 __global__ void split_bf16x2_kernel(const InT* __restrict__ src, int rows, int K, int64_t ld, int64_t ks,
                                     double scale, int Kp, __nv_bfloat16* __restrict__ dst) {
     const int gpr = Kp / 8;     // groups of 8 per row
     const int64_t total = (int64_t)rows * gpr;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(g / gpr), k0 = (int)(g % gpr) * 8;
+        const int r = total < (1ll << 31) ? (int)((unsigned)g / (unsigned)gpr) : (int)(g / gpr);
+        const int k0 = (int)(g - (int64_t)r * gpr) * 8;
         const InT* row = src + (int64_t)r * ld;
         __align__(16) __nv_bfloat16 hi[8], lo[8];
+        __align__(16) InT v[8];
+        if (VEC && k0 + 8 <= K) {
+            constexpr int n = 16 / (int)sizeof(InT);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int k = k0 + i;
-            const double x = k < K ? (double)__ldg(row + (int64_t)k * ks) * scale : 0.0;
-            hi[i] = __float2bfloat16_rn((float)x);
-            lo[i] = __float2bfloat16_rn((float)(x - (double)__bfloat162float(hi[i])));
+            for (int i = 0; i < 8; i += n)
+                *reinterpret_cast<uint4*>(v + i) = __ldg(reinterpret_cast<const uint4*>(row + k0 + i));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = k0 + i < K ? __ldg(row + (int64_t)(k0 + i) * ks) : InT(0);
+        }
+        if (std::is_same<InT, float>::value && scale == 1.0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {   // x - hi is exact in float32
+                const float x = (float)v[i];
+                hi[i] = __float2bfloat16_rn(x);
+                lo[i] = __float2bfloat16_rn(x - __bfloat162float(hi[i]));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const double x = k0 + i < K ? (double)v[i] * scale : 0.0;
+                hi[i] = __float2bfloat16_rn((float)x);
+                lo[i] = __float2bfloat16_rn((float)(x - (double)__bfloat162float(hi[i])));
+            }
         }
         __nv_bfloat16* d = dst + (int64_t)r * 2 * Kp + k0;
         *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(hi);
@@ -620,14 +643,19 @@ VTB_API int vtb_split_bf16x2(const void* src, int src_f32, int rows, int K, int6
     const int Kp = ceil_div(K, kTcBK) * kTcBK;
     const int64_t total = (int64_t)rows * (Kp / 8);
     const int blocks = (int)std::min<int64_t>(ceil_div(total, 256), 16 * kNumSMs);
-    if (src_f32)
-        split_bf16x2_kernel<float><<<blocks, 256, 0, as_stream(stream)>>>(
-            reinterpret_cast<const float*>(src), rows, K, ld, k_stride, scale, Kp,
-            reinterpret_cast<__nv_bfloat16*>(dst));
-    else
-        split_bf16x2_kernel<double><<<blocks, 256, 0, as_stream(stream)>>>(
-            reinterpret_cast<const double*>(src), rows, K, ld, k_stride, scale, Kp,
-            reinterpret_cast<__nv_bfloat16*>(dst));
+    const bool vec = k_stride == 1 && ((uintptr_t)src & 15) == 0 && (ld * (src_f32 ? 4 : 8)) % 16 == 0;
+    cudaStream_t s = as_stream(stream);
+    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(dst);
+    auto go = [&](auto kernel, auto* p) { kernel<<<blocks, 256, 0, s>>>(p, rows, K, ld, k_stride, scale, Kp, d); };
+    if (src_f32) {
+        const float* p = reinterpret_cast<const float*>(src);
+        if (vec) go(split_bf16x2_kernel<float, true>, p);
+        else go(split_bf16x2_kernel<float, false>, p);
+    } else {
+        const double* p = reinterpret_cast<const double*>(src);
+        if (vec) go(split_bf16x2_kernel<double, true>, p);
+        else go(split_bf16x2_kernel<double, false>, p);
+    }
     return launch_status();
 }
 

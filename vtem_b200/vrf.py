@@ -260,7 +260,11 @@ class vrf_cs(vrf):
 
 def _project(V, rf, alpha, P_expected, out_layout, precision):
     """alpha * V rf^T, (frames, N) or (N, frames) (vrf.py:264-292)."""
-    V = _dev(V).reshape(V.shape[0], -1)
+    # the split reads float32 frames as they are (float32 -> float64 is exact:
+    # the same operands as from a float64 copy)
+    single = precision == "bf16x3" and (V.dtype == torch.float32 if isinstance(V, torch.Tensor)
+                                        else np.asarray(V).dtype == np.float32)
+    V = _dev(V, torch.float32 if single else F64).reshape(V.shape[0], -1)
     F, P = V.shape
     if P != P_expected:
         raise ValueError("video frame size does not match the RF grid")
