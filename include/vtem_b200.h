@@ -447,6 +447,14 @@ int vtb_sym_factor(void* M, int64_t ld, int K, int mode, double rcond, void* wor
 /* x = M^-1 x (float64 x) with a factor of vtb_sym_factor of the same mode. */
 int vtb_sym_potrs(const void* Mfac, int64_t ld, double* x, int K, int mode, void* work, int64_t work_bytes,
                   void* stream);
+/* x = M^-1 x in float64 by a Cholesky factorisation in place (lower factor),
+ * factor and forward solve in one cooperative launch, the backward solve in a
+ * second.  flag and pivots as vtb_sym_factor (3: a bounded wait ran out; M and
+ * x are then undefined).  work: vtb_sym_chol_solve_bytes(K) bytes, 256-byte
+ * aligned. */
+int64_t vtb_sym_chol_solve_bytes(int K);
+int vtb_sym_chol_solve(double* M, int64_t ld, int K, double* x, double rcond, void* work, int64_t work_bytes,
+                       int32_t* flag, double* pivots, void* stream);
 /* One system, multi-CTA: x = L^-T L^-1 x (x float64, float32 arithmetic) with
  * a float32 factor of vtb_sym_factor (mode 2).  CTA j owns rows 64j..64j+63;
  * the forward and backward solves hand rows on through per-CTA flags

@@ -88,6 +88,8 @@ SIGNATURES = {
     "vtb_sym_workspace": [I, I, P],
     "vtb_sym_factor": [P, L, I, I, D, P, L, P, P, P],
     "vtb_sym_potrs": [P, L, P, I, I, P, L, P],
+    "vtb_sym_chol_solve_bytes": [I],  # restype int64, set in lib()
+    "vtb_sym_chol_solve": [P, L, I, P, D, P, L, P, P, P],
     "vtb_sym_dinv": [P, L, I, P, P],
     "vtb_sym_potrs_flags_bytes": [I],  # restype int64, set in lib()
     "vtb_sym_potrs_flags": [P, L, P, I, P, P, L, P, P],
@@ -148,7 +150,7 @@ def lib():
             f.argtypes = args
             f.restype = ctypes.c_int
         for name in ("vtb_sym_dinv_floats", "vtb_tc_group_bytes", "vtb_sym_potrs_flags_bytes", "vtb_chol_dinv_floats",
-                     "vtb_chol_work_bytes", "vtb_chol_inverse_floats", "vtb_chol_solve_inverse_bytes", "vtb_chol_batch_bytes"):
+                     "vtb_sym_chol_solve_bytes", "vtb_chol_work_bytes", "vtb_chol_inverse_floats", "vtb_chol_solve_inverse_bytes", "vtb_chol_batch_bytes"):
             getattr(l, name).argtypes = [ctypes.c_int]
             getattr(l, name).restype = ctypes.c_int64
         l.vtb_status_string.argtypes = [ctypes.c_int]

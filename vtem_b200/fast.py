@@ -50,6 +50,10 @@ C128 = torch.complex128
 # Cholesky is trusted only when the pivot spread is this far below 1/rcond
 # (a window with pivot spread 1.6e5 had condition number 1.2e10).
 CHOL_MARGIN = 1e4
+# float64 Cholesky solves up to this size take the tile kernel; tiles against
+# cuSOLVER (factor and solves, us): K = 25 24 / 50, 261 98 / 201, 979 270 / 595,
+# 1921 558 / 1129, 3001 1037 / 1747, 5001 2972 / 3425, 7001 7950 / 7381
+CHOL_TILES_MAX = 5120
 # accepted mixed solves: estimated relative error left after the last sweep
 MIXED_TOL = 1e-8
 
@@ -103,13 +107,16 @@ class CoeffDecoder(object):
         self.a = torch.empty((self.K,), dtype=C128, device=device)
         self.kept = torch.zeros(1, dtype=torch.int32, device=device)
         # real form: Mr (float64), right-hand side, iterate, correction
-        self.Mr = torch.empty((self.K, self.K), dtype=F64, device=device)
+        # K is odd: the float64 Cholesky solve takes columns of K + 1 (16-byte aligned)
+        self._Mr_store = torch.empty(self.K * (self.K + 1), dtype=F64, device=device)
+        self.Mr = self._Mr_store[:self.K * self.K].view(self.K, self.K)
         self.br = torch.empty((self.K,), dtype=F64, device=device)
         self.xr = torch.empty((self.K,), dtype=F64, device=device)
         self.rr = torch.empty((self.K,), dtype=F64, device=device)
         # status words read once per solve: [flag (int32), min pivot^2, max
         # pivot^2, sweep correction ratios x4, tensor-core error (int32)]
         self.stat = torch.zeros(8, dtype=F64, device=device)
+        self._chol64 = None
         self.last_ratios = []
         self._work = {}
         self.last_solver = None
@@ -409,15 +416,10 @@ class CoeffDecoder(object):
         self._build_M(s)
         call("vtb_coeff_realify_vec", dptr(self.b), K, 1, dptr(self.br), s)
         for i, mode in enumerate(modes):
-            call("vtb_coeff_realify", dptr(self.M), K, K, dptr(self.Mr), K, 1, s)
-            work = self._workspace(mode)
             if mode == 1:
-                self.stat.zero_()
-                call("vtb_sym_factor", dptr(self.Mr), K, K, 1, self.rcond * CHOL_MARGIN, dptr(work), work.numel(),
-                     self._stat_ptr(0), self._stat_ptr(1), s)
-                self.xr.copy_(self.br)
-                call("vtb_sym_potrs", dptr(self.Mr), K, dptr(self.xr), K, 1, dptr(work), work.numel(), s)
-                flag, piv, _, _ = self._read_stat()
+                flag, piv = self._chol_tiles(s) if K <= CHOL_TILES_MAX else (3, None)
+                if flag == 3:            # larger, or a wait of the tile solve ran out
+                    flag, piv = self._chol_library(s)
                 self.last_pivots = piv
                 if flag == 0:
                     call("vtb_coeff_unrealify_vec", dptr(self.xr), K, 1, dptr(self.a), 0, s)
@@ -427,6 +429,8 @@ class CoeffDecoder(object):
                 if i + 1 < len(modes):
                     continue
                 raise VtbError("vtb_sym_factor", VTB_NOT_CONVERGED)
+            call("vtb_coeff_realify", dptr(self.M), K, K, dptr(self.Mr), K, 1, s)
+            work = self._workspace(mode)
             rng = np.zeros(2, np.float64)
             call("vtb_sym_pinv", dptr(self.Mr), K, dptr(self.br), dptr(self.xr), K, self.rcond, dptr(work),
                  work.numel(), dptr(self.kept), rng.ctypes.data, s)
@@ -434,6 +438,28 @@ class CoeffDecoder(object):
             self.last_pivots = (float(rng[0]), float(rng[1]))
             self.last_solver = "eig"
             return
+
+    def _chol_tiles(self, s):
+        """xr = M^-1 br by the tile Cholesky; (flag, pivots), flag 3 when it gave up."""
+        K = self.K
+        if self._chol64 is None:
+            self._chol64 = torch.empty(int(lib().vtb_sym_chol_solve_bytes(K)), dtype=torch.uint8, device=self.M.device)
+        call("vtb_coeff_realify", dptr(self.M), K, K, dptr(self._Mr_store), K + 1, 1, s)
+        self.xr.copy_(self.br)
+        call("vtb_sym_chol_solve", dptr(self._Mr_store), K + 1, K, dptr(self.xr), self.rcond * CHOL_MARGIN,
+             dptr(self._chol64), self._chol64.numel(), self._stat_ptr(0), self._stat_ptr(1), s)
+        return self._read_stat()[:2]
+
+    def _chol_library(self, s):
+        """The same by cuSOLVER's factorisation and solves."""
+        K, work = self.K, self._workspace(1)
+        call("vtb_coeff_realify", dptr(self.M), K, K, dptr(self.Mr), K, 1, s)
+        self.stat.zero_()
+        call("vtb_sym_factor", dptr(self.Mr), K, K, 1, self.rcond * CHOL_MARGIN, dptr(work), work.numel(),
+             self._stat_ptr(0), self._stat_ptr(1), s)
+        self.xr.copy_(self.br)
+        call("vtb_sym_potrs", dptr(self.Mr), K, dptr(self.xr), K, 1, dptr(work), work.numel(), s)
+        return self._read_stat()[:2]
 
     def lambda_max(self, iters=40):
         """Largest eigenvalue of the float64 real system Mr (that of the
