@@ -28,21 +28,22 @@
 // every fragment read conflict-free.  Every wait is bounded: after the limit
 // the call is marked aborted (flag 3) and all CTAs return.
 //
-// The backward solve x = L^-T y is a second launch, one CTA per block row: a
-// lane keeps row r's partial sums of 8 columns over all blocks below, so only
-// the last block's product, one reduction over the warp and the product with
-// L_JJ^-T lie between two hand-offs; the hand-off is the value itself (readers
-// poll the words, which start as all ones).
+// The triangular solves are a second launch, one CTA per block row: the partial
+// sums over the blocks before stay in registers, so only the last block's
+// product, one reduction and the product with L_JJ^-1 lie between two
+// hand-offs; the hand-off is the value itself (readers poll the words, which
+// start as all ones).  Several solves, forward and backward in turn, run in one
+// launch, each reading the words of the one before.
 //
 // Bound: latency, the workers' more than the panel's: of a step's 16,000 cycles at
 // K = 979 the panel takes 9,000, and a tile passes two publications and two
 // products of workers between the steps that produce its operands and the one
 // that needs it.  Factor and solves, cuSOLVER -> here (us): K = 261 201 -> 98, 979
-// 595 -> 270, 1921 1129 -> 558, 3001 1747 -> 1037.  Columns that do not start
+// 595 -> 269, 1921 1129 -> 552, 3001 1747 -> 1024.  Columns that do not start
 // on 16 bytes are loaded entry by entry (679 us at 979).  Two and one CTAs per SM:
 // 271 and 289 us at 979, 1375 and 2246 at 3001; warp 3 publishing and writing
 // instead of taking a share of the products: 283 us at 979.
-#include "common.cuh"
+#include "chol_f64.cuh"
 
 #include <algorithm>
 
@@ -444,15 +445,19 @@ __device__ bool d_task(const DCholCtx& c, DCholSmem& sm, int I, int J, int type)
     return true;
 }
 
-__global__ void __launch_bounds__(kDThreads) chol64_kernel(DCholCtx c) {
-    extern __shared__ __align__(16) uint8_t d_smem[];
-    DCholSmem& sm = *reinterpret_cast<DCholSmem*>(d_smem);
-    if (blockIdx.x == 0) {
+struct DCholPair {
+    DCholCtx c[2];
+    int split;           // CTAs of the first system
+};
+
+// one system's CTAs: rank 0 the diagonal, the others workers
+__device__ __forceinline__ void d_system(const DCholCtx& c, DCholSmem& sm, int rank, int ctas) {
+    if (rank == 0) {
         d_diagonal(c, sm);
         return;
     }
-    const int W = gridDim.x - 1;
-    int t = blockIdx.x - 1, first = 0;      // tasks before group g
+    const int W = ctas - 1;
+    int t = rank - 1, first = 0;      // tasks before group g
     for (int g = 0; g <= c.T - 2; ++g) {
         const int n = d_group(c.T, g), n0 = c.T - g - 1;
         for (; t < first + n; t += W) {
@@ -465,132 +470,208 @@ __global__ void __launch_bounds__(kDThreads) chol64_kernel(DCholCtx c) {
     }
 }
 
-// ------------------------------------------------------------------ x = L^-T y
+__global__ void __launch_bounds__(kDThreads, kDPerSM) chol64_kernel(DCholCtx c) {
+    extern __shared__ __align__(16) uint8_t d_smem[];
+    d_system(c, *reinterpret_cast<DCholSmem*>(d_smem), blockIdx.x, gridDim.x);
+}
+
+__global__ void __launch_bounds__(kDThreads, kDPerSM) chol64_pair_kernel(const __grid_constant__ DCholPair pair) {
+    extern __shared__ __align__(16) uint8_t d_smem[];
+    const bool second = (int)blockIdx.x >= pair.split;
+    d_system(pair.c[second], *reinterpret_cast<DCholSmem*>(d_smem), blockIdx.x - (second ? pair.split : 0),
+             second ? gridDim.x - pair.split : pair.split);
+}
+
+// ------------------------------------------------------------------ triangular solves
 constexpr unsigned long long kDEmpty = 0xffffffffffffffffull;   // no result has these bits (see the store)
 
-__global__ void __launch_bounds__(kDThreads) chol64_back_kernel(DCholCtx c, unsigned long long* xo) {
+// the word at p once it is written
+__device__ __forceinline__ double d_value(const DCholCtx& c, const unsigned long long* p) {
+    const volatile unsigned long long* src = p;
+    unsigned long long v = *src;
+    for (unsigned it = 0; v == kDEmpty; v = *src)
+        if (++it > c.limit || *(volatile int*)c.abort_word != 0) {
+            atomicExch(c.abort_word, 1);
+            atomicMax(c.status, 3);
+            break;
+        }
+    return __longlong_as_double((long long)v);
+}
+
+// Phase p of np: block J's solution into out (and, in the last phase, x); in
+// is the phase before, null for x itself.
+__global__ void __launch_bounds__(kDThreads) chol64_solve_kernel(DCholCtx c, unsigned long long* words, int backward,
+                                                                 int np) {
     __shared__ double s_v[kDT], s_p[4][kDT];
+    const unsigned full = 0xffffffffu;
     const int T = c.T, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    for (int J = T - 1 - (int)blockIdx.x; J >= 0; J -= gridDim.x) {
-        // L_JJ^-1's rows 8w.. (column t = lane)
-        double di[8];
+    for (int p = 0; p < np; ++p, backward ^= 1) {
+        unsigned long long* out = words + (int64_t)p * T * kDT;
+        const unsigned long long* in = p ? out - (int64_t)T * kDT : nullptr;
+        auto rhs = [&](int i) -> double { return in ? d_value(c, in + i) : i < c.K ? __ldcg(c.x + i) : 0.0; };
+        for (int b = blockIdx.x; b < T; b += gridDim.x) {
+            const int J = backward ? T - 1 - b : b;
+            // L_JJ^-1: lane = its column t of the rows 8w.. (backward), its row of the columns 8w.. (forward)
+            const double* D = c.Dinv + (int64_t)J * kDT * kDT;
+            double di[8], l[8], acc[8] = {};
 #pragma unroll
-        for (int q = 0; q < 8; ++q) di[q] = __ldcg(c.Dinv + (int64_t)J * kDT * kDT + (8 * w + q) * kDT + lane);
-        double acc[8] = {}, l[8];
-        auto fetch = [&](int I) {          // rows I*32 + lane of the columns J*32 + 8w..
-            const int gr = I * kDT + lane;
+            for (int q = 0; q < 8; ++q) di[q] = __ldcg(backward ? D + (8 * w + q) * kDT + lane : D + lane * kDT + 8 * w + q);
+            const int other = backward ? T - 1 : 0, last = backward ? J + 1 : J - 1, step = backward ? -1 : 1;
+            const int n = b;                       // blocks before J in this order
+            auto fetch = [&](int I) {              // backward: tile (I, J); forward: tile (J, I)
+                const int gr = (backward ? I : J) * kDT + lane, gc0 = (backward ? J : I) * kDT + 8 * w;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int gc = J * kDT + 8 * w + q;
-                l[q] = gr < c.K && gc < c.K ? __ldcg(c.A + (int64_t)gc * c.ld + gr) : 0.0;
-            }
-        };
-        if (T - 1 > J) fetch(T - 1);
-        for (int I = T - 1; I > J; --I) {
-            const volatile unsigned long long* src = xo + I * kDT + lane;
-            unsigned long long v = *src;
-            for (unsigned it = 0; v == kDEmpty; v = *src)
-                if (++it > c.limit || *(volatile int*)c.abort_word != 0) {
-                    atomicExch(c.abort_word, 1);
-                    atomicMax(c.status, 3);
-                    break;
+                for (int q = 0; q < 8; ++q)
+                    l[q] = gr < c.K && gc0 + q < c.K ? __ldcg(c.A + (int64_t)(gc0 + q) * c.ld + gr) : 0.0;
+            };
+            if (n) fetch(other);
+            for (int k = 0, I = other; k < n; ++k, I += step) {
+                if (backward) {                    // acc[q]: this row's part of column 8w + q
+                    const double xv = d_value(c, out + I * kDT + lane);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) acc[q] = fma(l[q], xv, acc[q]);
+                } else {                           // acc[q]: row `lane`, column 8w + q
+                    const double xv = d_value(c, out + I * kDT + 8 * w + (lane & 7));
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) acc[q] = fma(l[q], __shfl_sync(full, xv, q), acc[q]);
                 }
-            const double xv = __longlong_as_double((long long)v);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) acc[q] = fma(l[q], xv, acc[q]);
-            if (I - 1 > J) fetch(I - 1);
-        }
-        // sums over the warp's lanes: 8 columns -> lane 4q holds column q
-        const unsigned full = 0xffffffffu;
-#pragma unroll
-        for (int h = 4; h >= 1; h >>= 1) {
-            const bool up = lane & (h * 4);
-#pragma unroll
-            for (int q = 0; q < h; ++q) {
-                const double give = up ? acc[q] : acc[q + h], keep = up ? acc[q + h] : acc[q];
-                acc[q] = keep + __shfl_xor_sync(full, give, h * 4);
+                if (I != last) fetch(I + step);
             }
-        }
-        acc[0] += __shfl_xor_sync(full, acc[0], 2);
-        acc[0] += __shfl_xor_sync(full, acc[0], 1);
-        if ((lane & 3) == 0) {
-            const int j = 8 * w + (lane >> 2), gc = J * kDT + j;
-            s_v[j] = (gc < c.K ? __ldcg(c.x + gc) : 0.0) - acc[0];
-        }
-        __syncwarp();
-        double p0 = 0.0, p1 = 0.0;
+            if (backward) {
+                // sums over the warp's lanes: 8 columns -> lane 4q holds column q
 #pragma unroll
-        for (int q = 0; q < 8; q += 2) {
-            p0 = fma(di[q], s_v[8 * w + q], p0);
-            p1 = fma(di[q + 1], s_v[8 * w + q + 1], p1);
+                for (int h = 4; h >= 1; h >>= 1) {
+                    const bool up = lane & (h * 4);
+#pragma unroll
+                    for (int q = 0; q < h; ++q) {
+                        const double give = up ? acc[q] : acc[q + h], keep = up ? acc[q + h] : acc[q];
+                        acc[q] = keep + __shfl_xor_sync(full, give, h * 4);
+                    }
+                }
+                acc[0] += __shfl_xor_sync(full, acc[0], 2);
+                acc[0] += __shfl_xor_sync(full, acc[0], 1);
+                if ((lane & 3) == 0) {
+                    const int j = 8 * w + (lane >> 2);
+                    s_v[j] = rhs(J * kDT + j) - acc[0];
+                }
+                __syncwarp();
+            } else {
+                s_p[w][lane] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+                __syncthreads();
+                if (lane < 8) {                    // each warp the entries it reads below
+                    const int j = 8 * w + lane;
+                    s_v[j] = rhs(J * kDT + j) - ((s_p[0][j] + s_p[1][j]) + (s_p[2][j] + s_p[3][j]));
+                }
+                __syncthreads();
+            }
+            double p0 = 0.0, p1 = 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                p0 = fma(di[q], s_v[8 * w + q], p0);
+                p1 = fma(di[q + 1], s_v[8 * w + q + 1], p1);
+            }
+            s_p[w][lane] = p0 + p1;
+            __syncthreads();
+            if (w == 0) {
+                const double r = (s_p[0][lane] + s_p[1][lane]) + (s_p[2][lane] + s_p[3][lane]);
+                unsigned long long bits = (unsigned long long)__double_as_longlong(r);
+                if (bits == kDEmpty) bits = 0x7ff8000000000000ull;
+                *reinterpret_cast<volatile unsigned long long*>(out + J * kDT + lane) = bits;
+                if (p + 1 == np && J * kDT + lane < c.K) c.x[J * kDT + lane] = r;
+            }
+            __syncthreads();
         }
-        s_p[w][lane] = p0 + p1;
-        __syncthreads();
-        if (w == 0) {
-            const double r = (s_p[0][lane] + s_p[1][lane]) + (s_p[2][lane] + s_p[3][lane]);
-            unsigned long long bits = (unsigned long long)__double_as_longlong(r);
-            if (bits == kDEmpty) bits = 0x7ff8000000000000ull;
-            *reinterpret_cast<volatile unsigned long long*>(xo + J * kDT + lane) = bits;
-            if (J * kDT + lane < c.K) c.x[J * kDT + lane] = r;
-        }
-        __syncthreads();
     }
 }
 
 static int64_t d_al(int64_t b) { return (b + 255) & ~(int64_t)255; }
 
+// [Dinv][flags][abort word 256][words of the solves' phases]
+int64_t chol64_bytes(int K) {
+    if (K <= 0) return 0;
+    const int64_t T = ceil_div(K, kDT);
+    return d_al(T * kDT * kDT * 8) + d_al((T + 1) * T * 4) + 256 + d_al(kChol64Phases * T * kDT * 8);
+}
+
+static DCholCtx d_context(const Chol64System& y) {
+    DCholCtx c;
+    c.A = y.A;
+    c.ld = y.ld;
+    c.K = y.K;
+    c.T = ceil_div(y.K, kDT);
+    c.x = y.x;
+    char* p = reinterpret_cast<char*>(y.work);
+    c.Dinv = reinterpret_cast<double*>(p);
+    p += d_al((int64_t)c.T * kDT * kDT * 8);
+    c.flag = reinterpret_cast<unsigned*>(p);
+    c.abort_word = reinterpret_cast<int*>(p + d_al((int64_t)(c.T + 1) * c.T * 4));
+    c.status = y.status;
+    c.piv = y.pivots;
+    c.rcond = y.rcond;
+    c.limit = wait_limit(kDSpin);
+    return c;
+}
+
+static int d_resident(const void* kernel, size_t smem, int* nsm, int* per_sm) {
+    int dev = 0, coop = 0;
+    VTB_CUDA_TRY(cudaGetDevice(&dev));
+    VTB_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    VTB_CUDA_TRY(cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev));
+    VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, kDThreads, smem));
+    return coop && *per_sm >= 1 ? VTB_OK : VTB_CUDA_ERR;
+}
+
+int chol64_factor(const Chol64System* systems, int n, cudaStream_t s) {
+    const size_t sm = sizeof(DCholSmem);
+    int nsm = 0, per_sm = 0;
+    const void* kernel = n == 1 ? (const void*)chol64_kernel : (const void*)chol64_pair_kernel;
+    const int st = d_resident(kernel, sm, &nsm, &per_sm);
+    if (st) return st;
+    const int room = std::min(per_sm, kDPerSM) * nsm / n;
+    DCholPair pair = {};
+    int ctas[2] = {0, 0};
+    for (int i = 0; i < n; ++i) {
+        DCholCtx& c = pair.c[i];
+        c = d_context(systems[i]);
+        int tasks = 0;
+        for (int g = 0; g <= c.T - 2; ++g) tasks += d_group(c.T, g);
+        ctas[i] = 1 + std::max(1, std::min(room - 1, tasks));
+        VTB_CUDA_TRY(cudaMemsetAsync(c.status, 0, 4, s));
+        VTB_CUDA_TRY(cudaMemsetAsync(c.flag, 0, (size_t)(d_al((int64_t)(c.T + 1) * c.T * 4) + 256), s));
+    }
+    pair.split = ctas[0];
+    void* args[] = {n == 1 ? (void*)&pair.c[0] : (void*)&pair};
+    VTB_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(ctas[0] + ctas[1]), dim3(kDThreads), args, sm,
+                                             s));
+    return launch_status();
+}
+
+int chol64_solve(const Chol64System& system, bool backward_first, int phases, cudaStream_t s) {
+    int nsm = 0, per_sm = 0;
+    const int st = d_resident((const void*)chol64_solve_kernel, 0, &nsm, &per_sm);
+    if (st) return st;
+    DCholCtx c = d_context(system);
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(c.abort_word) + 256);
+    VTB_CUDA_TRY(cudaMemsetAsync(words, 0xff, (size_t)phases * c.T * kDT * 8, s));
+    int first = backward_first;
+    void* args[] = {(void*)&c, (void*)&words, (void*)&first, (void*)&phases};
+    VTB_CUDA_TRY(cudaLaunchCooperativeKernel((void*)chol64_solve_kernel, dim3(std::min(c.T, per_sm * nsm)),
+                                             dim3(kDThreads), args, 0, s));
+    return launch_status();
+}
+
 }  // namespace vtb
 
 using namespace vtb;
 
-VTB_API int64_t vtb_sym_chol_solve_bytes(int K) {
-    if (K <= 0) return 0;
-    const int64_t T = ceil_div(K, kDT);
-    return d_al(T * kDT * kDT * 8) + d_al((T + 1) * T * 4) + 256 + d_al(T * kDT * 8);
-}
+VTB_API int64_t vtb_sym_chol_solve_bytes(int K) { return chol64_bytes(K); }
 
 VTB_API int vtb_sym_chol_solve(double* M, int64_t ld, int K, double* x, double rcond, void* work, int64_t work_bytes,
                                int32_t* flag, double* pivots, void* stream) {
     VTB_CHECK_ARG(K > 0 && ld >= K && M && x && work && flag);
-    VTB_CHECK_ARG(work_bytes >= vtb_sym_chol_solve_bytes(K) && ((uintptr_t)work & 255) == 0);
-    int dev = 0, coop = 0, nsm = 0, per_sm = 0, back = 0;
-    VTB_CUDA_TRY(cudaGetDevice(&dev));
-    VTB_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    VTB_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const size_t sm = sizeof(DCholSmem);
-    VTB_CUDA_TRY(cudaFuncSetAttribute(chol64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chol64_kernel, kDThreads, sm));
-    VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&back, chol64_back_kernel, kDThreads, 0));
-    if (!coop || per_sm < 1 || back < 1) return VTB_CUDA_ERR;
-    const int T = ceil_div(K, kDT);
-    int tasks = 0;
-    for (int g = 0; g <= T - 2; ++g) tasks += d_group(T, g);
-    cudaStream_t s = as_stream(stream);
-    char* p = reinterpret_cast<char*>(work);
-    DCholCtx c;
-    c.A = M;
-    c.ld = ld;
-    c.K = K;
-    c.T = T;
-    c.x = x;
-    c.Dinv = reinterpret_cast<double*>(p);
-    p += d_al((int64_t)T * kDT * kDT * 8);
-    c.flag = reinterpret_cast<unsigned*>(p);
-    c.abort_word = reinterpret_cast<int*>(p + d_al((int64_t)(T + 1) * T * 4));
-    unsigned long long* xo =
-        reinterpret_cast<unsigned long long*>(p + d_al((int64_t)(T + 1) * T * 4) + 256);
-    c.status = flag;
-    c.piv = pivots;
-    c.rcond = rcond;
-    c.limit = wait_limit(kDSpin);
-    VTB_CUDA_TRY(cudaMemsetAsync(flag, 0, 4, s));
-    VTB_CUDA_TRY(cudaMemsetAsync(c.flag, 0, (size_t)(d_al((int64_t)(T + 1) * T * 4) + 256), s));
-    VTB_CUDA_TRY(cudaMemsetAsync(xo, 0xff, (size_t)T * kDT * 8, s));
-    void* args[] = {(void*)&c};
-    const int grid = 1 + std::max(1, std::min(std::min(per_sm, kDPerSM) * nsm - 1, tasks));
-    VTB_CUDA_TRY(cudaLaunchCooperativeKernel((void*)chol64_kernel, dim3(grid), dim3(kDThreads), args, sm, s));
-    void* bargs[] = {(void*)&c, (void*)&xo};
-    VTB_CUDA_TRY(cudaLaunchCooperativeKernel((void*)chol64_back_kernel, dim3(std::min(T, back * nsm)), dim3(kDThreads),
-                                             bargs, 0, s));
-    return launch_status();
+    VTB_CHECK_ARG(work_bytes >= chol64_bytes(K) && ((uintptr_t)work & 255) == 0);
+    const Chol64System y{M, ld, K, x, work, flag, pivots, rcond};
+    const int st = chol64_factor(&y, 1, as_stream(stream));
+    return st ? st : chol64_solve(y, true, 1, as_stream(stream));
 }

@@ -27,17 +27,19 @@
 // far, lives on the device (accepted counts vary); the product runs over the
 // host's upper bound, the columns beyond k being zero.
 //
+// B and the shifted B are factorised side by side by the float64 tile Cholesky
+// and B^-2 applied in one launch of its triangular solves (two library
+// factorisations and eight library solves took 447 us of 1002 at r = 261).
 // Measured at n = 1900, r = 261 (the small configuration): 21.0 ms with the
-// eigendecomposition, 1.1 ms here; n = 24000, r = 1921: 6.9 s and 22 ms.  A
+// eigendecomposition, 0.75 ms here; n = 24000, r = 1921: 6.9 s and 19 ms.  A
 // matrix of full rank is refused after the first steps (by the trace its
 // columns have taken) or at n/2 columns: 0.2 ms lost of 3.3 at n = 300, 0.4 of
 // 28 at n = 2000.
-#include <cusolverDn.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
 
+#include "chol_f64.cuh"
 #include "common.cuh"
 #include "gemm_f64.cuh"
 
@@ -415,33 +417,28 @@ __global__ void __launch_bounds__(1024) pc_probe_kernel(const double* __restrict
 }
 
 // |B|_inf by rows into the state (a maximum of non-negative doubles orders like their bits)
-__global__ void __launch_bounds__(256) pc_norm_kernel(const double* __restrict__ B, int r, PcState* __restrict__ st) {
+__global__ void __launch_bounds__(256) pc_norm_kernel(const double* __restrict__ B, int r, int ldb,
+                                                      PcState* __restrict__ st) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= r) return;
     double s = 0.0;
-    for (int j = lane; j < r; j += 32) s += fabs(B[(int64_t)i * r + j]);
+    for (int j = lane; j < r; j += 32) s += fabs(B[(int64_t)i * ldb + j]);
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0)
         atomicMax(reinterpret_cast<unsigned long long*>(&st->norm), (unsigned long long)__double_as_longlong(s));
 }
 
-__global__ void pc_shift_kernel(const double* __restrict__ B, int r, double rcond, const PcState* __restrict__ st,
-                                double* __restrict__ B2) {
+__global__ void pc_shift_kernel(const double* __restrict__ B, int r, int ldb, double rcond,
+                                const PcState* __restrict__ st, double* __restrict__ B2) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= (int64_t)r * r) return;
-    B2[e] = B[e] - (e / r == e % r ? rcond * st->norm : 0.0);
-}
-
-static cusolverDnHandle_t psd_handle(int dev) {
-    static thread_local cusolverDnHandle_t h[64] = {nullptr};
-    if (dev < 0 || dev >= 64) return nullptr;
-    if (!h[dev] && cusolverDnCreate(&h[dev]) != CUSOLVER_STATUS_SUCCESS) h[dev] = nullptr;
-    return h[dev];
+    if (e >= (int64_t)r * ldb) return;
+    B2[e] = e % ldb < r ? B[e] - (e / ldb == e % ldb ? rcond * st->norm : 0.0) : 0.0;
 }
 
 struct PsdWork {
     PcState* st;
-    double *d, *L, *LP, *C, *B, *B2, *v, *y, *t, *wk;
+    double *d, *L, *LP, *C, *B, *B2, *v, *y, *t, *z;
+    void *wk, *wk2;
     int64_t ldl, bytes;
     int cols;
 };
@@ -450,7 +447,7 @@ struct PsdWork {
 // the better one), at most kPcMaxRank, and kPcB of slack
 static int psd_cols(int n) { return (std::min(n / 2, kPcMaxRank) + 2 * kPcB - 1) / kPcB * kPcB; }
 
-static PsdWork psd_work(int n, int lwork, char* base) {
+static PsdWork psd_work(int n, char* base) {
     PsdWork w;
     int64_t off = 0;
     auto take = [&](int64_t doubles) {
@@ -470,14 +467,11 @@ static PsdWork psd_work(int n, int lwork, char* base) {
     w.v = take(2 * (int64_t)n);
     w.y = take(2 * (int64_t)n);
     w.t = take(2 * (int64_t)w.cols);
-    w.wk = take(lwork);
+    w.z = take(w.cols);
+    w.wk = take(chol64_bytes(w.cols) / 8);
+    w.wk2 = take(chol64_bytes(w.cols) / 8);
     w.bytes = off;
     return w;
-}
-
-static int psd_lwork(cusolverDnHandle_t h, int n, int* lwork) {
-    return cusolverDnDpotrf_bufferSize(h, CUBLAS_FILL_MODE_LOWER, psd_cols(n), nullptr, psd_cols(n), lwork) ==
-                   CUSOLVER_STATUS_SUCCESS ? VTB_OK : VTB_CUDA_ERR;
 }
 
 }  // namespace vtb
@@ -486,13 +480,7 @@ using namespace vtb;
 
 VTB_API int vtb_solve_psd_workspace(int n, int64_t* bytes) {
     VTB_CHECK_ARG(n > 0 && bytes);
-    int dev = 0, lwork = 0;
-    VTB_CUDA_TRY(cudaGetDevice(&dev));
-    cusolverDnHandle_t h = psd_handle(dev);
-    if (!h) return VTB_CUDA_ERR;
-    const int st = psd_lwork(h, n, &lwork);
-    if (st) return st;
-    *bytes = psd_work(n, lwork, nullptr).bytes;
+    *bytes = psd_work(n, nullptr).bytes;
     return VTB_OK;
 }
 
@@ -501,16 +489,10 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
     VTB_CHECK_ARG(n > 0 && ld >= n && G && q && c && work && accepted && ((uintptr_t)work & 255) == 0);
     *accepted = 0;
     if (!(rcond >= 100.0 * kPcTol) || !(rcond < 1.0)) return VTB_OK;   // the rule would keep noise
-    int dev = 0, lwork = 0;
-    VTB_CUDA_TRY(cudaGetDevice(&dev));
-    cusolverDnHandle_t h = psd_handle(dev);
-    if (!h) return VTB_CUDA_ERR;
-    int st = psd_lwork(h, n, &lwork);
-    if (st) return st;
-    const PsdWork w = psd_work(n, lwork, reinterpret_cast<char*>(work));
+    int st = VTB_OK;
+    const PsdWork w = psd_work(n, reinterpret_cast<char*>(work));
     VTB_CHECK_ARG(work_bytes >= w.bytes);
     cudaStream_t s = as_stream(stream);
-    if (cusolverDnSetStream(h, s) != CUSOLVER_STATUS_SUCCESS) return VTB_CUDA_ERR;
     VTB_CUDA_TRY(cudaMemsetAsync(w.L, 0, (size_t)n * w.ldl * 8, s));
     pc_init_kernel<<<1, 1024, 0, s>>>(G, ld, n, w.d, w.st);
     struct {
@@ -537,23 +519,24 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
     st = launch_status();
     if (st) return st;
     if (host.done != 1 || host.bad || host.k < 1) return VTB_OK;
-    const int r = host.k;
-    const GemmF64Args gb{r, r, n, w.L, 1, w.ldl, w.L, 1, w.ldl, w.B, r, 1, 1.0, 0.0};
+    const int r = host.k, ldb = r + (r & 1);      // columns on 16 bytes
+    const GemmF64Args gb{r, r, n, w.L, 1, w.ldl, w.L, 1, w.ldl, w.B, ldb, 1, 1.0, 0.0};
     st = gemm_f64(gb, s);
     if (st) return st;
-    pc_norm_kernel<<<ceil_div((int64_t)r * 32, 256), 256, 0, s>>>(w.B, r, w.st);
-    pc_shift_kernel<<<ceil_div((int64_t)r * r, 256), 256, 0, s>>>(w.B, r, rcond, w.st, w.B2);
+    pc_norm_kernel<<<ceil_div((int64_t)r * 32, 256), 256, 0, s>>>(w.B, r, ldb, w.st);
+    pc_shift_kernel<<<ceil_div((int64_t)r * ldb, 256), 256, 0, s>>>(w.B, r, ldb, rcond, w.st, w.B2);
     int* info = reinterpret_cast<int*>(reinterpret_cast<char*>(w.st) + offsetof(PcState, info));
-    if (cusolverDnDpotrf(h, CUBLAS_FILL_MODE_LOWER, r, w.B2, r, w.wk, lwork, info + 1) != CUSOLVER_STATUS_SUCCESS ||
-        cusolverDnDpotrf(h, CUBLAS_FILL_MODE_LOWER, r, w.B, r, w.wk, lwork, info) != CUSOLVER_STATUS_SUCCESS)
-        return VTB_CUDA_ERR;
-    int* unused = reinterpret_cast<int*>(w.wk);
-    // c (+)= L B^-1 B^-1 L^T x
+    // B for the solves, and B - rcond |B| I for the rule (its right-hand side, 0, is not used)
+    const Chol64System sys[2] = {{w.B, ldb, r, w.t, w.wk, info, nullptr, 0.0},
+                                 {w.B2, ldb, r, w.z, w.wk2, info + 1, nullptr, 0.0}};
+    VTB_CUDA_TRY(cudaMemsetAsync(w.z, 0, (size_t)r * 8, s));
+    // c (+)= L B^-1 B^-1 L^T x; the first time with the factorisation, which leaves the first forward solve done
     auto apply = [&](const double* x, int add) -> int {
         pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, x, w.t);
-        for (int i = 0; i < 2; ++i)
-            if (cusolverDnDpotrs(h, CUBLAS_FILL_MODE_LOWER, r, 1, w.B, r, w.t, r, unused) != CUSOLVER_STATUS_SUCCESS)
-                return VTB_CUDA_ERR;
+        const int f = add ? VTB_OK : chol64_factor(sys, 2, s);
+        if (f) return f;
+        const int g = chol64_solve(sys[0], !add, add ? 4 : 3, s);
+        if (g) return g;
         pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, c, add);
         return VTB_OK;
     };

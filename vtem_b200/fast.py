@@ -51,8 +51,8 @@ C128 = torch.complex128
 # (a window with pivot spread 1.6e5 had condition number 1.2e10).
 CHOL_MARGIN = 1e4
 # float64 Cholesky solves up to this size take the tile kernel; tiles against
-# cuSOLVER (factor and solves, us): K = 25 24 / 50, 261 98 / 201, 979 270 / 595,
-# 1921 558 / 1129, 3001 1037 / 1747, 5001 2972 / 3425, 7001 7950 / 7381
+# cuSOLVER (factor and solves, us): K = 25 24 / 50, 261 98 / 201, 979 269 / 595,
+# 1921 552 / 1129, 3001 1024 / 1747, 5001 2972 / 3425, 7001 7950 / 7381
 CHOL_TILES_MAX = 5120
 # accepted mixed solves: estimated relative error left after the last sweep
 MIXED_TOL = 1e-8
