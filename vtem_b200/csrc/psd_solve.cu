@@ -31,7 +31,7 @@
 // and B^-2 applied in one launch of its triangular solves (two library
 // factorisations and eight library solves took 447 us of 1002 at r = 261).
 // Measured at n = 1900, r = 261 (the small configuration): 21.0 ms with the
-// eigendecomposition, 0.75 ms here; n = 24000, r = 1921: 6.9 s and 19 ms.  A
+// eigendecomposition, 0.9 ms here; n = 24000, r = 1921: 6.9 s and 19 ms.  A
 // matrix of full rank is refused after the first steps (by the trace its
 // columns have taken) or at n/2 columns: 0.2 ms lost of 3.3 at n = 300, 0.4 of
 // 28 at n = 2000.
