@@ -58,6 +58,30 @@ def test_pivot_flags(K):
     assert _solve(D, b, K, rcond=1e-9)[2] == 0
 
 
+@pytest.mark.parametrize("K", [65, 261, 979])
+def test_tiles_of_the_call(K):
+    """Two systems solved in turn in the same buffers: a tile read before its
+    writer has published it would hold the other system's numbers."""
+    systems = [_spd(K, s) for s in (1, 2)]
+    ld = K + (K & 1)
+    A = torch.empty((K, ld), dtype=torch.float64, device="cuda")
+    x = torch.empty(K, dtype=torch.float64, device="cuda")
+    w = torch.empty(int(lib().vtb_sym_chol_solve_bytes(K)), dtype=torch.uint8, device="cuda")
+    flags = torch.zeros(100, dtype=torch.int32, device="cuda")
+    first, same = [], torch.ones((), dtype=torch.bool, device="cuda")
+    for i in range(100):
+        M, b = systems[i & 1]
+        A[:, :K] = M
+        x.copy_(b)
+        call("vtb_sym_chol_solve", dptr(A), ld, K, dptr(x), 1e-12, dptr(w), w.numel(), flags.data_ptr() + 4 * i, None,
+             stream_ptr())
+        if i < 2:
+            first.append((A[:, :K].clone(), x.clone()))
+        else:
+            same &= (A[:, :K] == first[i & 1][0]).all() & (x == first[i & 1][1]).all()
+    assert int(flags.abs().max()) == 0 and bool(same)
+
+
 def test_wait_limit_runs_out_and_recovers():
     M, b = _spd(979, 5)
     with _abi.wait_limit(1):

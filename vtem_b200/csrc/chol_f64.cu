@@ -327,6 +327,9 @@ __device__ void d_diagonal(const DCholCtx& c, DCholSmem& sm) {
                 ok = d_poll(c, c.flag + (k + 1) * T + k, 1u, more ? c.flag + (k + 1) * T + k + 1 : nullptr, 1u);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (lane == 0) sm.ok = ok;
+            // a shuffle exchanges registers only: this barrier orders every lane's
+            // loads of the two tiles after lane 0's acquire
+            __syncwarp();
             if (ok) {
                 d_load(c, X, k + 1, k, lane, 32);
                 if (more) d_load(c, Y, k + 1, k + 1, lane, 32);
