@@ -228,8 +228,9 @@ int vtb_solve_eq_sym(double* G, int64_t ld, const double* q, double* c, int n, d
 /* The same solve for a positive semidefinite G of rank at most about n/2 whose
  * eigenvalues all lie clear of the truncation (above rcond * max, or rounding
  * noise): c = G^+ q by a pivoted Cholesky G = L L^T and the r x r system
- * L^T L, without an eigendecomposition.  *accepted (host) is 1 when that was
- * certified; else 0, and the caller solves with vtb_solve_eq_sym: G (its lower
+ * L^T L, without an eigendecomposition.  *accepted (host) is 1 when G was found
+ * to be such a matrix (for an indefinite G by pseudo-random probes of
+ * G - L L^T); else 0, and the caller solves with vtb_solve_eq_sym: G (its lower
  * triangle is read) is not written either way.  *kept (device, may be NULL)
  * receives r.  Synchronises the stream. */
 int vtb_solve_psd_workspace(int n, int64_t* bytes);

@@ -91,3 +91,28 @@ def test_left_to_the_eigendecomposition(kind):
     assert kept == keep.sum()
     size = max(np.linalg.norm(want), 1e-300)
     assert np.linalg.norm(c.cpu().numpy().ravel() - want) <= 1e-9 * size
+
+
+@pytest.mark.parametrize("s,t", [(1, 1), (1, -1), (-1, 1), (-1, -1)])
+def test_cycle_behind_zero_diagonal(s, t):
+    """A four-cycle on rows of zero diagonal, the rest of low rank: no diagonal
+    entry shows its eigenvalues +-2a, and a vector of +-1 with v5 v6 = s and
+    v9 v10 = t lies in its null space."""
+    n, r = 320, 20
+    rng = np.random.default_rng(8)
+    A = rng.standard_normal((n, r))
+    A[[5, 6, 9, 10]] = 0.0
+    Q, _ = np.linalg.qr(A)
+    G = (Q * np.geomspace(1.0, 1e-2, r)) @ Q.T
+    G = 0.5 * (G + G.T)
+    for i, j, e in ((5, 9, 0.2), (5, 10, -0.2 * t), (6, 9, -0.2 * s), (6, 10, 0.2 * s * t)):
+        G[i, j] = G[j, i] = e
+    q = rng.standard_normal(n)
+    assert not _solve(G, q)[0]
+    c, kept = linalg.solve_eq_sym(torch.as_tensor(G, device="cuda"), torch.as_tensor(q, device="cuda").reshape(-1, 1),
+                                  rcond=RCOND, return_kept=True)
+    w, V = np.linalg.eigh(G)
+    keep = np.abs(w) > RCOND * np.abs(w).max()
+    want = V[:, keep] @ ((V[:, keep].T @ q) / np.abs(w[keep]))
+    assert kept == keep.sum() == r + 2
+    assert np.linalg.norm(c.cpu().numpy().ravel() - want) <= 1e-9 * np.linalg.norm(want)

@@ -9,11 +9,16 @@
 //   B = L^T L (r x r, the nonzero eigenvalues of G),
 //   G^+ q = L B^-1 B^-1 L^T q,  refined once with q - G c,
 // which is the reference's truncated pseudoinverse exactly when the rule
-// s > rcond * s_0 drops the noise and keeps the rest.  Both are certified:
-// B - rcond * |B|_inf I has a Cholesky factorisation (every eigenvalue of B
-// passes the rule), and the remainder G - L L^T is below it (by its trace, and
-// by its action on a fixed vector, as an indefinite G could hide from its
-// diagonal).  Anything else is left to the
+// s > rcond * s_0 drops the noise and keeps the rest.  Both are tested.
+// B - rcond * |B|_inf I has a Cholesky factorisation: every eigenvalue of B
+// passes the rule.  The remainder E = G - L L^T is below it: by its trace, which
+// decides for a semidefinite G, and, as an indefinite one can hide from its
+// diagonal, by |E v| for kPcProbes pseudo-random vectors v.  That part is
+// probabilistic: an eigenvalue e of E above the rule passes when its eigenvector
+// is nearly orthogonal to every v, |<v, u>| below 0.05 rule / e, under one
+// chance in 25 a vector.  The vectors' magnitudes vary and their seed is taken from G, so that
+// no pattern of entries cancels in all of them (signs alone miss a four-cycle
+// of +-a on rows of zero diagonal).  Anything else is left to the
 // eigendecomposition: *accepted = 0, G untouched.
 //
 // Pivots are taken kPcB at a time: candidates are the largest remaining
@@ -47,6 +52,7 @@ namespace vtb {
 
 constexpr int kPcB = 32;               // candidates (and at most as many pivots) per step
 constexpr int kPcMaxRank = 3072;       // columns the workspace holds at most
+constexpr int kPcProbes = 3;            // vectors the remainder is tried on
 constexpr double kPcKeep = 0.01;       // accepted pivots, relative to the largest remaining diagonal
 // pivots end here, relative to G's largest diagonal entry: the noise left by
 // the updates is mostly below 1e-13 (1.4e-14 absolute at n = 2000, r = 800), but
@@ -64,7 +70,7 @@ struct PcState {
     double trace0;                     // of G
     double R[kPcB * kPcB];             // factor of the accepted block, row-major lower
     double trace;                      // of the remainder G - L L^T
-    double probe, norm;                // |G v - L L^T v|_2; |B|_inf
+    double probe, norm;                // largest |G v - L L^T v|_2 of the probes; |B|_inf
     int info[2];
 };
 
@@ -295,7 +301,7 @@ __global__ void __launch_bounds__(64) pc_update_kernel(const double* __restrict_
     if (i < n) d[i] = own < kPcB ? 0.0 : d[i] - s;
 }
 
-// y_b = A^T x_b (row-major A, n x r) for one or two vectors: block of 32 columns x 32 row groups
+// y_b = A^T x_b (row-major A, n x r), b < gridDim.y: block of 32 columns x 32 row groups
 __global__ void __launch_bounds__(1024) pc_gemv_t_kernel(const double* __restrict__ A, int64_t ld, int n, int r,
                                                         const double* __restrict__ x, double* __restrict__ y) {
     __shared__ double part[32][33];
@@ -332,58 +338,63 @@ __global__ void __launch_bounds__(256) pc_gemv_kernel(const double* __restrict__
     if (lane == 0) *q = add ? *q + s : s;
 }
 
-// y_b = G x_b from G's lower triangle, b = 0, 1: the part left of the diagonal
+// y_b = G x_b from G's lower triangle, b < NV: the part left of the diagonal
 // by rows (one warp each) into y, then the part below it by columns added
+template <int NV>
 __global__ void __launch_bounds__(256) pc_symv_rows_kernel(const double* __restrict__ G, int64_t ld, int n,
                                                            const double* __restrict__ x, double* __restrict__ y) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
     const double* row = G + (int64_t)i * ld;
-    double s = 0.0, t = 0.0;
+    double s[NV] = {};
     for (int j = lane; j <= i; j += 32) {
         const double g = row[j];
-        s = fma(g, x[j], s);
-        t = fma(g, x[n + j], t);
+#pragma unroll
+        for (int b = 0; b < NV; ++b) s[b] = fma(g, x[(int64_t)b * n + j], s[b]);
     }
-    for (int o = 16; o; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    if (lane == 0) {
-        y[i] = s;
-        y[n + i] = t;
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+        for (int o = 16; o; o >>= 1) s[b] += __shfl_xor_sync(0xffffffffu, s[b], o);
+        if (lane == 0) y[(int64_t)b * n + i] = s[b];
     }
 }
 
+template <int NV>
 __global__ void __launch_bounds__(512) pc_symv_cols_kernel(const double* __restrict__ G, int64_t ld, int n,
                                                            const double* __restrict__ x, double* __restrict__ y) {
-    __shared__ double ps[16][33], pt[16][33];
-    const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
-    double s = 0.0, t = 0.0;
+    __shared__ double part[NV][16][33];
+    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, g = threadIdx.x >> 5;
+    double s[NV] = {};
     if (c < n)
         for (int i = blockIdx.x * 32 + g; i < n; i += 16)
             if (i > c) {
                 const double v = G[(int64_t)i * ld + c];
-                s = fma(v, x[i], s);
-                t = fma(v, x[n + i], t);
+#pragma unroll
+                for (int b = 0; b < NV; ++b) s[b] = fma(v, x[(int64_t)b * n + i], s[b]);
             }
-    ps[g][threadIdx.x & 31] = s;
-    pt[g][threadIdx.x & 31] = t;
+#pragma unroll
+    for (int b = 0; b < NV; ++b) part[b][g][lane] = s[b];
     __syncthreads();
-    if (g == 0 && c < n) {
-        for (int k = 1; k < 16; ++k) {
-            s += ps[k][threadIdx.x & 31];
-            t += pt[k][threadIdx.x & 31];
-        }
-        y[c] += s;
-        y[n + c] += t;
+    if (g < NV && c < n) {
+        double t = 0.0;
+        for (int k = 0; k < 16; ++k) t += part[g][k][lane];
+        y[(int64_t)g * n + c] += t;
     }
 }
 
-// the probe vector: signs by a fixed integer hash
-__global__ void pc_signs_kernel(double* __restrict__ v, int n) {
+// the probes: entries of either sign and magnitudes 0.5 to 1.5, from the splitmix64
+// generator (Steele, Lea, Flood 2014) seeded by G's trace and largest diagonal entry
+__global__ void pc_probes_kernel(double* __restrict__ v, int n, const PcState* __restrict__ st) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = __popc((unsigned)i * 2654435761u ^ ((unsigned)i >> 7)) & 1 ? 1.0 : -1.0;
+    if (i >= kPcProbes * n) return;
+    unsigned long long z = (unsigned long long)__double_as_longlong(st->trace0) ^
+                           ((unsigned long long)__double_as_longlong(st->maxd0) << 1);
+    z += 0x9e3779b97f4a7c15ull * (unsigned long long)(i + 1);
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    z ^= z >> 31;
+    const double m = 0.5 + (double)(z >> 12) * 0x1p-52;
+    v[i] = z & 1 ? m : -m;
 }
 
 // res = q - y
@@ -393,10 +404,13 @@ __global__ void pc_residual_kernel(const double* __restrict__ q, const double* _
     if (i < n) res[i] = q[i] - y[i];
 }
 
-// st->probe = |y - z|_2, st->trace = sum of |d| (one block)
+// st->probe = the largest |y_b - z_b|_2 (raised to it; one block per probe),
+// st->trace = sum of |d|
 __global__ void __launch_bounds__(1024) pc_probe_kernel(const double* __restrict__ y, const double* __restrict__ z,
                                                         const double* __restrict__ d, int n, PcState* __restrict__ st) {
     __shared__ double sm[32], tm[32];
+    y += (int64_t)blockIdx.x * n;
+    z += (int64_t)blockIdx.x * n;
     double s = 0.0, t = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         s = fma(y[i] - z[i], y[i] - z[i], s);
@@ -416,8 +430,10 @@ __global__ void __launch_bounds__(1024) pc_probe_kernel(const double* __restrict
             s += sm[w];
             t += tm[w];
         }
-        st->probe = sqrt(s);
-        st->trace = t;
+        // (non-negative doubles, and a NaN above them, order like their bits)
+        atomicMax(reinterpret_cast<unsigned long long*>(&st->probe),
+                  (unsigned long long)__double_as_longlong(fabs(sqrt(s))));
+        if (blockIdx.x == 0) st->trace = t;
     }
 }
 
@@ -469,9 +485,9 @@ static PsdWork psd_work(int n, char* base) {
     w.C = take((int64_t)n * kPcB);
     w.B = take((int64_t)w.cols * w.cols);
     w.B2 = take((int64_t)w.cols * w.cols);
-    w.v = take(2 * (int64_t)n);
-    w.y = take(2 * (int64_t)n);
-    w.t = take(2 * (int64_t)w.cols);
+    w.v = take((1 + kPcProbes) * (int64_t)n);
+    w.y = take((1 + kPcProbes) * (int64_t)n);
+    w.t = take(kPcProbes * (int64_t)w.cols);
     w.z = take(w.cols);
     w.wk = take(chol64_bytes(w.cols) / 8);
     w.wk2 = take(chol64_bytes(w.cols) / 8);
@@ -546,14 +562,15 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
         return VTB_OK;
     };
     if ((st = apply(q, 0))) return st;
-    // one pass over G for the refinement (x = c) and the probe (x = signs)
+    // one pass over G for the refinement (x = c) and the probes
+    constexpr int nv = 1 + kPcProbes;
     VTB_CUDA_TRY(cudaMemcpyAsync(w.v, c, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
-    pc_signs_kernel<<<ceil_div(n, 256), 256, 0, s>>>(w.v + n, n);
-    pc_symv_rows_kernel<<<ceil_div((int64_t)n * 32, 256), 256, 0, s>>>(G, ld, n, w.v, w.y);
-    pc_symv_cols_kernel<<<ceil_div(n, 32), 512, 0, s>>>(G, ld, n, w.v, w.y);
-    pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, w.v + n, w.t);
-    pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, w.v + n, 0);
-    pc_probe_kernel<<<1, 1024, 0, s>>>(w.y + n, w.v + n, w.d, n, w.st);
+    pc_probes_kernel<<<ceil_div((int64_t)kPcProbes * n, 256), 256, 0, s>>>(w.v + n, n, w.st);
+    pc_symv_rows_kernel<nv><<<ceil_div((int64_t)n * 32, 256), 256, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_symv_cols_kernel<nv><<<ceil_div(n, 32), 512, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), kPcProbes), 1024, 0, s>>>(w.L, w.ldl, n, r, w.v + n, w.t);
+    pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), kPcProbes), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, w.v + n, 0);
+    pc_probe_kernel<<<kPcProbes, 1024, 0, s>>>(w.y + n, w.v + n, w.d, n, w.st);
     pc_residual_kernel<<<ceil_div(n, 256), 256, 0, s>>>(q, w.y, w.v, n);
     if ((st = apply(w.v, 1))) return st;
     PcState end;
