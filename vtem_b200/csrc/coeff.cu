@@ -968,7 +968,7 @@ static void launch_ws(int My, int blocks, size_t smf, cudaStream_t s, const doub
                       int Mx, int Mt, double W, double t0, double dt, int Nt, int Px, int Py, int Px1, int Py1, int YS,
                       OutT* u, cudaError_t* err) {
     auto go = [&](auto kern) {
-        *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
+        *err = allow_call_smem(kern);
         if (*err == cudaSuccess)
             kern<<<blocks, kWsThreads, smf, s>>>(a, smap, Ks, Mx, Mt, W, t0, dt, Nt, Px, Py, Px1, Py1, YS, u);
     };
@@ -1043,7 +1043,7 @@ VTB_API int vtb_coeff_synthesize(const double* a, const int32_t* smap, int Ks, i
         const size_t smf = (size_t)(Ks * Kt + kFoldFrames * (Kt + Ky * Kx)) * sizeof(double2) +
                            (size_t)(kFoldFrames * H * (2 + 4 * Mx) + kWsSlots * 16 * kFoldXS + 16 * YS) *
                                sizeof(double);
-        VTB_CHECK_ARG(smf <= 200 * 1024);
+        VTB_CHECK_ARG(smf <= kCallSmem);
         const int blocks = (int)std::min<int64_t>(Nt, 2 * kNumSMs);
         cudaError_t err = cudaSuccess;
         if (out_f32)
@@ -1059,19 +1059,15 @@ VTB_API int vtb_coeff_synthesize(const double* a, const int32_t* smap, int Ks, i
         // fused half-spectrum kernel (A_work unused)
         const size_t smh = (size_t)(Kx * Px + Ks * Kt + kHalfFrames * (Kt + Ky * Kx)) * sizeof(double2) +
                            (size_t)(kHalfFrames * Ky * Px + Ky * Py) * sizeof(double);
-        VTB_CHECK_ARG(smh <= 200 * 1024);
+        VTB_CHECK_ARG(smh <= kCallSmem);
         const int blocks = (int)std::min<int64_t>(ceil_div(Nt, kHalfFrames), 2 * kNumSMs);
         if (out_f32) {
-            if (smh > 48 * 1024)
-                VTB_CUDA_TRY(cudaFuncSetAttribute(synth_half_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)smh));
+            if (smh > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(synth_half_kernel<float>));
             synth_half_kernel<float><<<blocks, 256, smh, s>>>(reinterpret_cast<const double2*>(a), smap, Ks, Mx, My, Mt,
                                                               W, t0, dt, Nt, Px, Py, Px1, Py1,
                                                               reinterpret_cast<float*>(u));
         } else {
-            if (smh > 48 * 1024)
-                VTB_CUDA_TRY(cudaFuncSetAttribute(synth_half_kernel<double>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smh));
+            if (smh > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(synth_half_kernel<double>));
             synth_half_kernel<double><<<blocks, 256, smh, s>>>(reinterpret_cast<const double2*>(a), smap, Ks, Mx, My,
                                                                Mt, W, t0, dt, Nt, Px, Py, Px1, Py1,
                                                                reinterpret_cast<double*>(u));
@@ -1084,16 +1080,14 @@ VTB_API int vtb_coeff_synthesize(const double* a, const int32_t* smap, int Ks, i
     int st = launch_status();
     if (st) return st;
     const size_t sm = (size_t)(Kx * Px + Ky * Py + Ky * Kx + Ky * Px) * sizeof(double2);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
+    VTB_CHECK_ARG(sm <= kCallSmem);
     const int blocks = ceil_div(Nt, kSynthFrames);
     if (out_f32) {
-        if (sm > 48 * 1024)
-            VTB_CUDA_TRY(cudaFuncSetAttribute(synth_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(synth_kernel<float>));
         synth_kernel<float><<<blocks, 256, sm, s>>>(reinterpret_cast<const double2*>(A_work), smap, Ks, Mx, My, Px,
                                                    Py, Px1, Py1, Nt, reinterpret_cast<float*>(u));
     } else {
-        if (sm > 48 * 1024)
-            VTB_CUDA_TRY(cudaFuncSetAttribute(synth_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(synth_kernel<double>));
         synth_kernel<double><<<blocks, 256, sm, s>>>(reinterpret_cast<const double2*>(A_work), smap, Ks, Mx, My, Px,
                                                     Py, Px1, Py1, Nt, reinterpret_cast<double*>(u));
     }
@@ -1179,13 +1173,9 @@ VTB_API int vtb_coeff_synthesize_noalloc(const double* a, const int32_t* smap, i
     const int Kt = 2 * Mt + 1;
     const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
     const size_t sm = (size_t)(Kx * Px + Ky * Py + Ky * Kx + Ky * Px) * sizeof(double2);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
-    if (sm > 48 * 1024) {
-        if (out_f32)
-            VTB_CUDA_TRY(cudaFuncSetAttribute(synth_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        else
-            VTB_CUDA_TRY(cudaFuncSetAttribute(synth_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    }
+    VTB_CHECK_ARG(sm <= kCallSmem);
+    if (sm > 48 * 1024)
+        VTB_CUDA_TRY(out_f32 ? allow_call_smem(synth_kernel<float>) : allow_call_smem(synth_kernel<double>));
     const int chunk = (int)std::min<int64_t>(kNoAllocScratchElems / Ks, (int64_t)Nt);
     const int64_t frame = (int64_t)Px * Py;
     for (int f0 = 0; f0 < Nt; f0 += chunk) {

@@ -24,6 +24,17 @@ uint32_t wait_limit(uint32_t default_polls);
 
 constexpr int kNumSMs = 148;
 
+// Dynamic shared memory allowed to the kernels whose need goes with the call's
+// sizes.  The limit is an attribute of the kernel, shared by every host thread:
+// set to one call's need, another thread's smaller call could lower it before the
+// launch that needs it (which is then refused), so it is only ever set to this.
+constexpr size_t kCallSmem = 200 * 1024;
+
+template <typename Kernel>
+inline cudaError_t allow_call_smem(Kernel* kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCallSmem);
+}
+
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // lower_bound of v in the sorted a[0..n) by one full warp: 32-way probes

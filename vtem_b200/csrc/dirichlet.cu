@@ -598,10 +598,10 @@ VTB_API int vtb_dirichlet_coeffs(const double* rf, int N, int LPy, int LPx, int6
     // (256 x 256: 74 KB, three blocks per SM); longer sides and more bins take the general kernel
     const int Xp = (LPx + 7) & ~7, Yp = (LPy + 15) & ~15;
     const size_t smm = (size_t)(2 * Yp + (LPx == LPy && Mx == My ? 0 : Xp)) * kDfS * sizeof(double);
-    if (Kx <= 16 && Ky <= 16 && smm <= 200 * 1024) {
+    if (Kx <= 16 && Ky <= 16 && smm <= kCallSmem) {
         const bool vec = LPx % 2 == 0 && rf_ld % 2 == 0 && ((uintptr_t)rf & 15) == 0;
         auto kernel = vec ? ds_mma_kernel<true> : ds_mma_kernel<false>;
-        VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
+        VTB_CUDA_TRY(allow_call_smem(kernel));
         const int per_sm = smm > 100 * 1024 ? 1 : smm > 56 * 1024 ? 2 : 4;
         kernel<<<std::min(N, per_sm * kNumSMs), kDfWarps * 32, smm, as_stream(stream)>>>(
             rf, rf_ld, N, LPy, LPx, Mx, My, dxdy, reinterpret_cast<double2*>(Ds));
@@ -609,9 +609,8 @@ VTB_API int vtb_dirichlet_coeffs(const double* rf, int N, int LPy, int LPx, int6
     }
     const size_t sm = (size_t)(LPx + LPy) * sizeof(double2) + (size_t)kDsRows * LPx * sizeof(double) +
                       (size_t)kDsRows * Kx * sizeof(double2);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
-    if (sm > 48 * 1024)
-        VTB_CUDA_TRY(cudaFuncSetAttribute(ds_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    VTB_CHECK_ARG(sm <= kCallSmem);
+    if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(ds_kernel));
     ds_kernel<<<N, 256, sm, as_stream(stream)>>>(rf, rf_ld, LPy, LPx, Mx, My, dxdy,
                                                  reinterpret_cast<double2*>(Ds));
     return launch_status();
@@ -626,12 +625,10 @@ VTB_API int vtb_dirich_space(const double* Ds, int N, int Mx, int My, int Px, in
     VTB_CHECK_ARG(Ds && out);
     const int Ky = 2 * My + 1;
     const size_t base = (size_t)Ky * (Px + Py) * sizeof(double2);
-    VTB_CHECK_ARG(base <= 200 * 1024);
-    const int table = base + (size_t)Px1 * sizeof(double2) <= 200 * 1024;
+    VTB_CHECK_ARG(base <= kCallSmem);
+    const int table = base + (size_t)Px1 * sizeof(double2) <= kCallSmem;
     const size_t sm = base + (table ? (size_t)Px1 * sizeof(double2) : 0);
-    if (sm > 48 * 1024)
-        VTB_CUDA_TRY(
-            cudaFuncSetAttribute(dirich_space_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(dirich_space_kernel));
     dirich_space_kernel<<<N, 256, sm, as_stream(stream)>>>(reinterpret_cast<const double2*>(Ds), Mx, My, Px, Py,
                                                           Px1, Py1, table, out);
     return launch_status();

@@ -980,10 +980,8 @@ VTB_API int vtb_sym_potrs_batched(const void* descs, int batch, int Kmax, void* 
     if (batch == 0) return VTB_OK;
     VTB_CHECK_ARG(descs);
     const size_t sm = (size_t)(Kmax + 32) * sizeof(float);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
-    if (sm > 48 * 1024)
-        VTB_CUDA_TRY(
-            cudaFuncSetAttribute(trsv_pair_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    VTB_CHECK_ARG(sm <= kCallSmem);
+    if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(trsv_pair_batched_kernel));
     trsv_pair_batched_kernel<<<batch, kTrsvThreads, sm, as_stream(stream)>>>(reinterpret_cast<const TrsvDesc*>(descs));
     return launch_status();
 }

@@ -324,12 +324,16 @@ VTB_API int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double
     int blocks = (K + rows - 1) / rows;
     size_t sm = (size_t)K * 8 + (size_t)rows * K * 8;
     int cache = 1;
+    cudaFuncAttributes fa;
+    VTB_CUDA_TRY(cudaFuncGetAttributes(&fa, rnn_coeff_kernel));
+    smem_max -= (int)fa.sharedSizeBytes;
     if (sm > (size_t)smem_max) {
         cache = 0;
         sm = (size_t)K * 8;
         VTB_CHECK_ARG(sm <= (size_t)smem_max);
     }
-    VTB_CUDA_TRY(cudaFuncSetAttribute(rnn_coeff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    // (the limit is the kernel's, not the call's: always the same one)
+    VTB_CUDA_TRY(cudaFuncSetAttribute(rnn_coeff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     int per_sm = 0;
     VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rnn_coeff_kernel, kRnnThreads, sm));
     if (per_sm * nsm < blocks) return VTB_CUDA_ERR;

@@ -375,9 +375,8 @@ static int launch_basis(const double* a, const int32_t* smap, int Ks, int Mx, in
     VTB_CHECK_ARG((int64_t)Mx * Px1 < (1LL << 30) && (int64_t)My * Py1 < (1LL << 30));
     const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
     const size_t sm = (size_t)(Kx * kBX + 2 * Ky * kBX + Ky * kBY + 2 * Ky * Kx) * sizeof(double2);
-    VTB_CHECK_ARG(sm <= 200 * 1024);
-    if (sm > 48 * 1024)
-        VTB_CUDA_TRY(cudaFuncSetAttribute(basis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    VTB_CHECK_ARG(sm <= kCallSmem);
+    if (sm > 48 * 1024) VTB_CUDA_TRY(allow_call_smem(basis_kernel));
     dim3 grid(ceil_div(Px, kBX) * ceil_div(Py, kBY), Mt + 1);
     basis_kernel<<<grid, kBX * kBY, sm, stream>>>(reinterpret_cast<const double2*>(a), smap, Ks, Mx, My, Mt, Px, Py,
                                                   Px1, Py1, H, ldh);
