@@ -43,3 +43,37 @@ def test_uniform_reconstruction(N, Py, Px, Mt, n, t0, Nt, order):
     size = np.bincount(ind, weights=term, minlength=N) @ np.abs(phi).reshape(N, -1)
     tol = np.finfo(np.float64).eps * (8 + Mt * W * (t0 + T + Nt * dt) + N + n) * size.max()
     assert np.abs(u - uo).max() <= tol
+
+
+@pytest.mark.parametrize("t0", [0.3, 5.0, -70.1])
+def test_times_are_those_of_arange(t0):
+    """np.arange steps by fl(t0 + dt) - t0; over many frames that is far from
+    dt.  Against the general kernel on arange's own times."""
+    N, Mt, n, Nt, dt = 9, 6, 60, 4000, 1e-4
+    rng = np.random.default_rng(3)
+    Wt = 2 * np.pi * 20
+    a = t0 + rng.uniform(0, 0.4, n)
+    b = a + rng.uniform(0.003, 0.05, n)
+    ind = np.sort(rng.integers(0, N, n)).astype(np.int32)
+    c, one, phi = rng.standard_normal(n), np.ones(N), rng.standard_normal((N, 6, 5))
+    cp = dirichlet.dirichlet(N, a, b, ind, one, one, one, one, Wt, Mt)
+    cp.d_q = torch.as_tensor(c, device="cuda").reshape(-1, 1)
+    frame = [t0, t0 + (Nt - 0.5) * dt]
+    u = cp.reconstruct(phi, frame, dt).cpu().numpy().reshape(Nt, -1)
+    t = np.arange(frame[0], frame[1], dt)
+    call = dirichlet.call
+    d = [torch.as_tensor(x, device="cuda") for x in (phi, a, b, c, ind, one, t)]
+    nb = np.zeros(1, np.int64)
+    call("vtb_reconstruct_workspace", N, len(t), Mt, nb.ctypes.data)
+    work = torch.empty(int(nb[0]), dtype=torch.uint8, device="cuda")
+    want = torch.empty((len(t), 30), dtype=torch.float64, device="cuda")
+    p = [x.data_ptr() for x in d]
+    call("vtb_reconstruct", p[0], N, 30, p[1], p[2], p[3], p[4], p[5], n, p[6], len(t), Mt, Wt / Mt, want.data_ptr(),
+         work.data_ptr(), work.numel(), dirichlet.stream_ptr())
+    assert u.shape == (Nt, 30)
+    # the rounding of the arguments m W t on both sides, and of two sums of N and n terms
+    W, m = Wt / Mt, np.arange(1, Mt + 1)
+    term = np.abs(c) * ((b - a) + (4 / W) * (1 / m).sum())
+    size = np.bincount(ind, weights=term, minlength=N) @ np.abs(phi).reshape(N, -1)
+    tol = 2 * np.finfo(np.float64).eps * (8 + Mt * W * (abs(t0) + 0.5) + N + n) * size.max()
+    assert np.abs(u - want.cpu().numpy()).max() <= tol

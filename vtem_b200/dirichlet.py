@@ -132,8 +132,10 @@ class dirichlet(object):
         if 1 <= self.Mt <= 10:
             call("vtb_reconstruct_uniform_workspace", N, Py * Px, self.Mt, nbytes.ctypes.data)
             work = torch.empty(int(nbytes[0]), dtype=torch.uint8, device="cuda")
+            # arange's own step, fl(t0 + dt) - t0: its samples drift from t0 + i dt
+            step = float(t[1] - t[0]) if len(t) > 1 else float(dt)
             call("vtb_reconstruct_uniform", dptr(dirich), N, Py * Px, dptr(tk1), dptr(tk2), dptr(c), dptr(ind),
-                 dptr(self.d_norm), self.size, float(time_frame[0]), float(dt), len(t), self.Mt, self.Wt / self.Mt,
+                 dptr(self.d_norm), self.size, float(time_frame[0]), step, len(t), self.Mt, self.Wt / self.Mt,
                  dptr(u), dptr(work), int(nbytes[0]), stream_ptr())
             return u
         d_t = _dev(t)
