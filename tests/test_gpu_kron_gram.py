@@ -31,3 +31,19 @@ def test_kron_gram(N, Ks, Kt):
     assert np.all(np.abs(got - want) <= 8 * np.finfo(np.float64).eps * (N + 4) * size)
     assert np.array_equal(got, np.conj(got.T))
     assert np.all(M.cpu().numpy()[:, K:] == 7.0 + 7.0j)
+
+
+def test_more_pairs_than_a_grid_dimension():
+    """2.2 million pairs of spatial indices (65,536 rows of 32 and more)."""
+    Ks = 2100
+    rng = np.random.default_rng(2)
+    d = torch.as_tensor(rng.standard_normal(Ks) + 1j * rng.standard_normal(Ks), device="cuda")
+    W = torch.full((1, 1, 1), 1.5, dtype=torch.complex128, device="cuda")
+    g = torch.full((1, 1), 0.5 - 0.25j, dtype=torch.complex128, device="cuda")
+    M = torch.zeros((Ks, Ks), dtype=torch.complex128, device="cuda")
+    b = torch.empty(Ks, dtype=torch.complex128, device="cuda")
+    call("vtb_coeff_gram", dptr(d), 1, Ks, dptr(W), dptr(g), 1, dptr(M), Ks, dptr(b), stream_ptr())
+    want = 1.5 * torch.outer(d, d.conj())
+    eps = np.finfo(np.float64).eps
+    assert bool(((M.T - want).abs() <= 4 * eps * want.abs()).all())
+    assert bool(((b - d * g[0, 0]).abs() <= 4 * eps * b.abs()).all())

@@ -9,8 +9,8 @@
 // all entries (1.9 ms at N = 1024, Ks = 113, Kt = 17 out of the FMA pipe;
 // 8.1 GFLOP and 0.37 ms here), bound by the float64 rate.
 //
-// A CTA forms kPairs pairs x kCols entries.  The pair products are formed on
-// the way into shared memory (4 operations against 2 kCols products each), the
+// A CTA forms TP pairs x TE entries.  The pair products are formed on
+// the way into shared memory (4 operations against 2 TE products each), the
 // temporal entries arrive by cp.async; slabs of 16 neurons, the pair operand
 // double-buffered through registers.  A product's 16 rows are the real parts
 // of 8 pairs and their imaginary parts, so that a lane ends up with the four
@@ -53,8 +53,11 @@ __global__ void __launch_bounds__(kKgThreads) kron_gram_kernel(const double2* __
     const int fr = lane >> 2, fk = lane & 3;
     const int64_t pairs = (int64_t)Ks * (Ks + 1) / 2;
     const int entries = Kt * (Kt + 1) / 2, KK = Kt * Kt;
-    const int64_t p0 = (int64_t)blockIdx.y * TP;
-    const int e0 = blockIdx.x * TE;
+    // the tiles of one row of pairs follow each other (the pairs alone can exceed
+    // the 65,535 of the grid's other dimensions: Ks > 2047)
+    const int et = (entries + TE - 1) / TE;
+    const int64_t p0 = (int64_t)(blockIdx.x / et) * TP;
+    const int e0 = blockIdx.x % et * TE;
     const int nk = (N + kKgK - 1) / kKgK;
     // this thread's pair (the same in every slab) and its neurons' stride
     const int q = tid % TP;
@@ -171,12 +174,11 @@ int kron_gram_f64(const double2* d, int N, int Ks, const double2* Wn, int Kt, do
     // while the larger tiles leave SMs without one
     const int64_t large = (pairs + 31) / 32 * ceil_div(entries, 32);
     if (large >= kNumSMs) {
-        if ((pairs + 31) / 32 > 65535) return VTB_BAD_ARG;
-        kron_gram_kernel<32, 32><<<dim3(ceil_div(entries, 32), ceil_div(pairs, 32)), kKgThreads, 0, s>>>(d, N, Ks, Wn, Kt,
-                                                                                                      M, ldm);
+        if (large > 0x7fffffff) return VTB_BAD_ARG;
+        kron_gram_kernel<32, 32><<<(unsigned)large, kKgThreads, 0, s>>>(d, N, Ks, Wn, Kt, M, ldm);
     } else {
-        kron_gram_kernel<16, 16><<<dim3(ceil_div(entries, 16), ceil_div(pairs, 16)), kKgThreads, 0, s>>>(d, N, Ks, Wn, Kt,
-                                                                                                      M, ldm);
+        kron_gram_kernel<16, 16><<<ceil_div(entries, 16) * ceil_div(pairs, 16), kKgThreads, 0, s>>>(d, N, Ks, Wn, Kt, M,
+                                                                                                    ldm);
     }
     return launch_status();
 }
