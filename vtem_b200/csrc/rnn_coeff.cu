@@ -9,12 +9,16 @@
 // ~25k at the GPU configuration).  In the real form (realsys.cu) this is
 // x <- x + dt*alpha*(br - Mr x), float64 like the reference.
 //
-// One cooperative launch runs every step: each CTA owns a block of rows of
-// Mr, kept in shared memory for the whole run when it fits (Mr is read from
-// HBM/L2 once, not once per step), stages the previous iterate in shared
-// memory, writes its rows of the next one, and meets the other CTAs at a
-// grid barrier.  The barrier's wait is bounded: a CTA that waits longer than
-// the limit sets *err and returns (the host reports VTB_TIMEOUT).
+// Two forms.  vtb_rnn_coeff_work, which the decoder uses, squares the update's
+// map first and takes what is left of the updates with the matrix in registers
+// (further down).  vtb_rnn_coeff takes every update one by one: in one cooperative launch
+// each CTA owns a block of rows of Mr, kept in shared memory for the whole run
+// when it fits (Mr is read from HBM/L2 once, not once per step), stages the
+// previous iterate in shared memory, writes its rows of the next one, and meets
+// the other CTAs at a grid barrier.  The barrier's wait is bounded: a CTA that
+// waits longer than the limit sets *err and returns (the host reports
+// VTB_TIMEOUT).  The same kernel follows the squared form (GUARD) and takes over
+// where the updates diverge.
 #include <algorithm>
 #include <mutex>
 
@@ -57,11 +61,24 @@ __device__ bool rnn_grid_barrier(unsigned* count, unsigned* gen, unsigned nblock
     return ok != 0;
 }
 
+// GUARD: x holds the iterate of the squared maps.  An update that contracts
+// never lengthens the residual br - Mr x (Mr symmetric: it multiplies each
+// eigenvector's part by 1 - dta lambda), so a residual longer than br shows
+// updates that diverge, where the squared maps' rounding grows with the number
+// of updates that each stands for instead of with its square root (402 updates,
+// dta lambda = 2.4 and 3.4: 1.8 times the sum of the updates' own rounding): all updates are then
+// taken here, from 0.  Else x stays.  (kRnnGrowth leaves room for the residual's own
+// rounding.)  Every CTA takes the sums over all rows in the same order and so
+// decides alike.  Measured at K = 1921: 14 us of 2590.
+constexpr double kRnnGrowth = 1.0 + 1e-6;
+
+template <bool GUARD>
 __global__ void __launch_bounds__(kRnnThreads) rnn_coeff_kernel(const double* __restrict__ Mr, int64_t ld,
                                                                 const double* __restrict__ br, double* xa,
                                                                 double* xb, int K, double dta, int updates,
                                                                 int rows_per_block, int cache_rows,
-                                                                unsigned* bar, int* err, unsigned limit) {
+                                                                unsigned* bar, int* err, unsigned limit,
+                                                                const double* x, double* res) {
     extern __shared__ double rnn_sm[];
     double* sx = rnn_sm;                 // K: previous iterate
     double* sM = rnn_sm + K;             // rows_per_block x K (when cache_rows)
@@ -73,10 +90,45 @@ __global__ void __launch_bounds__(kRnnThreads) rnn_coeff_kernel(const double* __
             const int r = (int)(e / K), j = (int)(e % K);
             sM[e] = Mr[(int64_t)(r0 + r) * ld + j];
         }
+    if (GUARD) {
+        __shared__ double sums[2][kRnnThreads / 32];
+        if (*(volatile int*)err) return;      // set by the launch before, or by a CTA that gave up: no one is waited for
+        for (int j = threadIdx.x; j < K; j += blockDim.x) sx[j] = __ldcg(x + j);
+        __syncthreads();
+        for (int r = r0 + warp; r < r1; r += nw) {
+            const double* row = cache_rows ? sM + (int64_t)(r - r0) * K : Mr + (int64_t)r * ld;
+            double s = 0.0;
+            for (int j = lane; j < K; j += 32) s = fma(row[j], sx[j], s);
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) __stcg(res + r, br[r] - s);
+        }
+        if (!rnn_grid_barrier(bar, bar + 1, gridDim.x, err, limit)) return;
+        double a = 0.0, b = 0.0;
+        for (int j = threadIdx.x; j < K; j += blockDim.x) {
+            const double r = __ldcg(res + j), q = br[j];
+            a = fma(r, r, a);
+            b = fma(q, q, b);
+        }
+        for (int o = 16; o; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        if (lane == 0) {
+            sums[0][warp] = a;
+            sums[1][warp] = b;
+        }
+        __syncthreads();
+        a = b = 0.0;
+        for (int k = 0; k < nw; ++k) {
+            a += sums[0][k];
+            b += sums[1][k];
+        }
+        if (a <= kRnnGrowth * b) return;      // (not with a NaN)
+    }
     for (int it = 0; it < updates; ++it) {
         const double* cur = (it & 1) ? xb : xa;
         double* nxt = (it & 1) ? xa : xb;
-        for (int j = threadIdx.x; j < K; j += blockDim.x) sx[j] = __ldcg(cur + j);
+        for (int j = threadIdx.x; j < K; j += blockDim.x) sx[j] = it ? __ldcg(cur + j) : 0.0;
         __syncthreads();
         for (int r = r0 + warp; r < r1; r += nw) {
             const double* row = cache_rows ? sM + (int64_t)(r - r0) * K : Mr + (int64_t)r * ld;
@@ -309,23 +361,19 @@ static int rnn_device(int* nsm, int* smem_max) {
     return coop ? VTB_OK : VTB_CUDA_ERR;
 }
 
-// x (K doubles, device) receives the iterate after steps+1 updates from x = 0;
-// x_tmp (K doubles) and bar (2 unsigned + 1 int of scratch, 16 bytes) are
-// caller-owned scratch.  Replaces rnn3 + rnn3_update (vtem/neural_network.py:
-// 15-128) on the real coefficient system.  Synchronises nothing; an
-// exceeded barrier wait is reported by vtb_rnn_coeff_status.
-VTB_API int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double* x, double* x_tmp, int K,
-                          double dt_alpha, int steps, void* bar, void* stream) {
-    VTB_CHECK_ARG(K > 0 && ld >= K && steps >= 0 && Mr && br && x && x_tmp && bar);
-    int nsm = 0, smem_max = 0;
-    int st = rnn_device(&nsm, &smem_max);
-    if (st) return st;
+// One launch of rnn_coeff_kernel (bar: 2 unsigned, then the error word, zeroed by
+// the caller); VTB_BAD_ARG where K doubles exceed a block's shared memory.
+template <bool GUARD>
+static int launch_rnn_updates(const double* Mr, int64_t ld, const double* br, double* xa, double* xb, int K,
+                              double dt_alpha, int updates, unsigned* bar, const double* x, double* res, int nsm,
+                              int smem_max, cudaStream_t s) {
+    auto kernel = rnn_coeff_kernel<GUARD>;
     int rows = (K + nsm - 1) / nsm;
     int blocks = (K + rows - 1) / rows;
     size_t sm = (size_t)K * 8 + (size_t)rows * K * 8;
     int cache = 1;
     cudaFuncAttributes fa;
-    VTB_CUDA_TRY(cudaFuncGetAttributes(&fa, rnn_coeff_kernel));
+    VTB_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
     smem_max -= (int)fa.sharedSizeBytes;
     if (sm > (size_t)smem_max) {
         cache = 0;
@@ -333,26 +381,41 @@ VTB_API int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double
         VTB_CHECK_ARG(sm <= (size_t)smem_max);
     }
     // (the limit is the kernel's, not the call's: always the same one)
-    VTB_CUDA_TRY(cudaFuncSetAttribute(rnn_coeff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    VTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     int per_sm = 0;
-    VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rnn_coeff_kernel, kRnnThreads, sm));
+    VTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRnnThreads, sm));
     if (per_sm * nsm < blocks) return VTB_CUDA_ERR;
-    cudaStream_t s = as_stream(stream);
-    VTB_CUDA_TRY(cudaMemsetAsync(x, 0, (size_t)K * 8, s));
-    VTB_CUDA_TRY(cudaMemsetAsync(bar, 0, 16, s));
-    const int updates = steps + 1;
-    unsigned* b = reinterpret_cast<unsigned*>(bar);
-    int* err = reinterpret_cast<int*>(b + 2);
-    double* xa = x;
-    double* xb = x_tmp;
+    int* err = reinterpret_cast<int*>(bar + 2);
     unsigned limit = wait_limit(kRnnSpinLimit);
     void* args[] = {(void*)&Mr, (void*)&ld, (void*)&br, (void*)&xa, (void*)&xb, (void*)&K, (void*)&dt_alpha,
-                    (void*)&updates, (void*)&rows, (void*)&cache, (void*)&b, (void*)&err, (void*)&limit};
-    VTB_CUDA_TRY(cudaLaunchCooperativeKernel((void*)rnn_coeff_kernel, dim3(blocks), dim3(kRnnThreads), args, sm, s));
-    // the result is in xa after an even number of updates, else in xb
-    if (updates & 1) VTB_CUDA_TRY(cudaMemcpyAsync(x, x_tmp, (size_t)K * 8, cudaMemcpyDeviceToDevice, s));
+                    (void*)&updates, (void*)&rows, (void*)&cache, (void*)&bar, (void*)&err, (void*)&limit,
+                    (void*)&x, (void*)&res};
+    VTB_CUDA_TRY(cudaLaunchCooperativeKernel((void*)kernel, dim3(blocks), dim3(kRnnThreads), args, sm, s));
     return launch_status();
 }
+
+// x (K doubles, device) receives the iterate after steps+1 updates from x = 0;
+// x_tmp (K doubles) and bar (2 unsigned + 1 int of scratch, 16 bytes) are
+// caller-owned scratch.  Replaces rnn3 + rnn3_update (vtem/neural_network.py:
+// 15-128) on the real coefficient system.  Synchronises nothing; an
+// exceeded barrier wait is reported in bar's third word.
+VTB_API int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double* x, double* x_tmp, int K,
+                          double dt_alpha, int steps, void* bar, void* stream) {
+    VTB_CHECK_ARG(K > 0 && ld >= K && steps >= 0 && Mr && br && x && x_tmp && bar);
+    int nsm = 0, smem_max = 0;
+    int st = rnn_device(&nsm, &smem_max);
+    if (st) return st;
+    cudaStream_t s = as_stream(stream);
+    VTB_CUDA_TRY(cudaMemsetAsync(bar, 0, 16, s));
+    const int updates = steps + 1;
+    // the last of an even number of updates writes the first buffer
+    double* xa = updates & 1 ? x_tmp : x;
+    double* xb = updates & 1 ? x : x_tmp;
+    return launch_rnn_updates<false>(Mr, ld, br, xa, xb, K, dt_alpha, updates, reinterpret_cast<unsigned*>(bar), nullptr,
+                                     nullptr, nsm, smem_max, s);
+}
+
+constexpr int kRnnGuardMax = 28000;
 
 // Workspace of vtb_rnn_coeff_work, every part on 256 bytes: status words,
 // packets, two of S and x, two of P (rows padded to 16 bytes).
@@ -383,12 +446,8 @@ static RnnWork rnn_work(int K, char* base) {
 
 // Squarings before the remaining updates run one by one, by cost in us: a
 // squaring with its pass over P (15 + K^3 / 2.5e7: 300 measured at
-// K = 1921) against an exchange (7.3 measured at K = 1921, 5.5 at 261).  None
-// where one CTA holds every row (K <= 2): its updates exchange nothing with
-// other SMs, and taken one by one their roundings do not add up in one
-// direction as a power's do where the updates diverge.
+// K = 1921) against an exchange (7.3 measured at K = 1921, 5.5 at 261).
 static int rnn_levels(int K, int updates) {
-    if (K <= 2) return 0;
     const double square = 15.0 + (double)K * K * K / 2.5e7, exchange = 7.3;
     int best = 0;
     for (int s = 1; (updates >> s) > 0; ++s)
@@ -411,7 +470,8 @@ VTB_API int vtb_rnn_coeff_work(const double* Mr, int64_t ld, const double* br, d
     int st = rnn_device(&nsm, &smem_max);
     if (st) return st;
     cudaStream_t s = as_stream(stream);
-    const int updates = steps + 1, levels = rnn_levels(K, updates);
+    // none where the guard's kernel could not hold the iterate in shared memory
+    const int updates = steps + 1, levels = K <= kRnnGuardMax ? rnn_levels(K, updates) : 0;
     VTB_CUDA_TRY(cudaMemsetAsync(w.status, 0, 16, s));
     rnn_map_kernel<<<dim3(ceil_div(K, 1024), K), 256, 0, s>>>(Mr, ld, br, K, dt_alpha, w.P[0], w.ldp, w.S[0], w.x[0]);
     int cur = 0;
@@ -425,13 +485,20 @@ VTB_API int vtb_rnn_coeff_work(const double* Mr, int64_t ld, const double* br, d
     const int left = updates >> levels, rows = ceil_div(K, nsm);
     double* xc = w.x[cur];
     const double *P = w.P[cur], *S = w.S[cur];
+    // the squared maps' iterate into x, and the check that it is no diverging one
+    double *res = w.S[cur ^ 1], *tmp = w.S[cur];
+    auto finish = [&](const double* from) -> int {
+        VTB_CUDA_TRY(cudaMemcpyAsync(x, from, (size_t)K * 8, cudaMemcpyDeviceToDevice, s));
+        if (levels == 0) return launch_status();
+        return launch_rnn_updates<true>(Mr, ld, br, updates & 1 ? tmp : x, updates & 1 ? x : tmp, K, dt_alpha, updates,
+                                        reinterpret_cast<unsigned*>(w.status), x, res, nsm, smem_max, s);
+    };
     // more rows than registers and shared memory hold: one pass over P an update
     if (rows > 13 || K > 4 * kRnnRegThreads || left == 1) {
         double* unused = w.S[cur ^ 1];
         for (int i = 0; i < left; ++i, cur ^= 1)
             rnn_apply_kernel<<<rows_grid, 256, 0, s>>>(P, w.ldp, K, S, w.x[cur], 1, unused, w.x[cur ^ 1]);
-        VTB_CUDA_TRY(cudaMemcpyAsync(x, w.x[cur], (size_t)K * 8, cudaMemcpyDeviceToDevice, s));
-        return launch_status();
+        return finish(w.x[cur]);
     }
     if (rows <= 2 && K <= kRnnRegThreads) st = launch_rnn_reg<2, 0, 1>(P, w.ldp, S, xc, K, left, w.packets, w.status + 2, nsm, s);
     else if (rows <= 4 && K <= 2 * kRnnRegThreads)
@@ -442,7 +509,5 @@ VTB_API int vtb_rnn_coeff_work(const double* Mr, int64_t ld, const double* br, d
         st = launch_rnn_reg<10, 0, 3>(P, w.ldp, S, xc, K, left, w.packets, w.status + 2, nsm, s);
     else
         st = launch_rnn_reg<10, 3, 4>(P, w.ldp, S, xc, K, left, w.packets, w.status + 2, nsm, s);
-    if (st) return st;
-    VTB_CUDA_TRY(cudaMemcpyAsync(x, xc, (size_t)K * 8, cudaMemcpyDeviceToDevice, s));
-    return launch_status();
+    return st ? st : finish(xc);
 }
