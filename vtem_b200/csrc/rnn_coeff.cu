@@ -69,7 +69,7 @@ __device__ bool rnn_grid_barrier(unsigned* count, unsigned* gen, unsigned nblock
 // dta lambda = 2.4 and 3.4: 1.8 times the sum of the updates' own rounding): all updates are then
 // taken here, from 0.  Else x stays.  (kRnnGrowth leaves room for the residual's own
 // rounding.)  Every CTA takes the sums over all rows in the same order and so
-// decides alike.  Measured at K = 1921: 14 us of 2590.
+// decides alike.  Measured at K = 1921: 16 us of 2600.
 constexpr double kRnnGrowth = 1.0 + 1e-6;
 
 template <bool GUARD>
@@ -85,19 +85,15 @@ __global__ void __launch_bounds__(kRnnThreads) rnn_coeff_kernel(const double* __
     const int r0 = blockIdx.x * rows_per_block;
     const int r1 = min(K, r0 + rows_per_block);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    if (cache_rows)
-        for (int64_t e = threadIdx.x; e < (int64_t)(r1 - r0) * K; e += blockDim.x) {
-            const int r = (int)(e / K), j = (int)(e % K);
-            sM[e] = Mr[(int64_t)(r0 + r) * ld + j];
-        }
     if (GUARD) {
         __shared__ double sums[2][kRnnThreads / 32];
         if (*(volatile int*)err) return;      // set by the launch before, or by a CTA that gave up: no one is waited for
         for (int j = threadIdx.x; j < K; j += blockDim.x) sx[j] = __ldcg(x + j);
         __syncthreads();
         for (int r = r0 + warp; r < r1; r += nw) {
-            const double* row = cache_rows ? sM + (int64_t)(r - r0) * K : Mr + (int64_t)r * ld;
+            const double* row = Mr + (int64_t)r * ld;
             double s = 0.0;
+#pragma unroll 8
             for (int j = lane; j < K; j += 32) s = fma(row[j], sx[j], s);
             for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (lane == 0) __stcg(res + r, br[r] - s);
@@ -125,6 +121,11 @@ __global__ void __launch_bounds__(kRnnThreads) rnn_coeff_kernel(const double* __
         }
         if (a <= kRnnGrowth * b) return;      // (not with a NaN)
     }
+    if (cache_rows)
+        for (int64_t e = threadIdx.x; e < (int64_t)(r1 - r0) * K; e += blockDim.x) {
+            const int r = (int)(e / K), j = (int)(e % K);
+            sM[e] = Mr[(int64_t)(r0 + r) * ld + j];
+        }
     for (int it = 0; it < updates; ++it) {
         const double* cur = (it & 1) ? xb : xa;
         double* nxt = (it & 1) ? xa : xb;
