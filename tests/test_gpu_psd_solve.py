@@ -116,3 +116,26 @@ def test_cycle_behind_zero_diagonal(s, t):
     want = V[:, keep] @ ((V[:, keep].T @ q) / np.abs(w[keep]))
     assert kept == keep.sum() == r + 2
     assert np.linalg.norm(c.cpu().numpy().ravel() - want) <= 1e-9 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n,r", [(400, 60), (1900, 261)])
+@pytest.mark.parametrize("cond", [1e2, 1e4, 1e6])
+def test_as_close_as_the_eigendecomposition(n, r, cond):
+    """Right-hand sides that weigh the spectrum differently, in G's range and
+    out of it: the error against the known solution, which the rounding of G
+    is part of on both sides, is that of the eigendecomposition."""
+    w = np.geomspace(1.0, 1.0 / cond, r)
+    G, Q = _matrix(n, w, n + r)
+    rng = np.random.default_rng(4)
+    for q in (Q @ (w * rng.standard_normal(r)), Q @ rng.standard_normal(r), rng.standard_normal(n)):
+        want = Q @ ((Q.T @ q) / w)
+        error = lambda c: np.linalg.norm(c - want) / np.linalg.norm(want)
+        ok, c, kept = _solve(G, q)
+        assert ok and kept == r
+        nb = np.zeros(1, np.int64)
+        call("vtb_solve_eq_sym_workspace", n, nb.ctypes.data)
+        work = torch.empty(int(nb[0]), dtype=torch.uint8, device="cuda")
+        Gd, qd = torch.as_tensor(G, device="cuda"), torch.as_tensor(q, device="cuda")
+        ce = torch.empty_like(qd)
+        call("vtb_solve_eq_sym", dptr(Gd), n, dptr(qd), dptr(ce), n, RCOND, dptr(work), work.numel(), None, stream_ptr())
+        assert error(c) <= 2 * error(ce.cpu().numpy())

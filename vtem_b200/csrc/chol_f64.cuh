@@ -17,7 +17,7 @@ struct Chol64System {
     double rcond;
 };
 
-constexpr int kChol64Phases = 4;
+constexpr int kChol64Phases = 6;      // at most
 
 int64_t chol64_bytes(int K);
 int chol64_factor(const Chol64System* systems, int n, cudaStream_t s);   // n = 1 or 2, factorised side by side

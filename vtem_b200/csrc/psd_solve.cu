@@ -7,7 +7,7 @@
 // matrix-vector products, to find a null space it drops.  Here instead
 //   G = L L^T,  L n x r,  by Cholesky with pivoting down to rounding noise,
 //   B = L^T L (r x r, the nonzero eigenvalues of G),
-//   G^+ q = L B^-1 B^-1 L^T q,  refined once with q - G c,
+//   c = G L B^-3 L^T q,  refined: c += L B^-3 L^T (G (q - G c)),
 // which is the reference's truncated pseudoinverse exactly when the rule
 // s > rcond * s_0 drops the noise and keeps the rest.  Both are tested.
 // B - rcond * |B|_inf I has a Cholesky factorisation: every eigenvalue of B
@@ -16,10 +16,22 @@
 // diagonal, by |E v| for kPcProbes pseudo-random vectors v.  That part is
 // probabilistic: an eigenvalue e of E above the rule passes when its eigenvector
 // is nearly orthogonal to every v, |<v, u>| below 0.05 rule / e, under one
-// chance in 25 a vector.  The vectors' magnitudes vary and their seed is taken from G, so that
-// no pattern of entries cancels in all of them (signs alone miss a four-cycle
-// of +-a on rows of zero diagonal).  Anything else is left to the
+// chance in 25 a vector.  The vectors' magnitudes vary and their seed is taken
+// from G, so that no pattern of entries cancels in all of them (signs alone miss
+// a four-cycle of +-a on rows of zero diagonal).  Anything else is left to the
 // eigendecomposition: *accepted = 0, G untouched.
+//
+// In exact arithmetic G L B^-3 L^T = L B^-2 L^T = G^+.  The range of the computed
+// L is off that of G by about sqrt(n k) eps |diag G| / s_r (the sums of k products
+// behind every column), several times the error of an eigenvector.  A product
+// with G returns the solution to G's own range, and takes the part of the
+// residual outside it away, at an error of eps |G| each.  One refinement does
+// until the condition number nears 1e7; more are taken while the last was above
+// kPcConverged, and a solve that does not settle is refused.  Relative error of c
+// against the known solution, for the spectra 1..1/cond of n = 1900, r = 261 and a q
+// outside the range: by L B^-2 L^T refined with q - G c 1.3e-13 at cond = 1e2 and
+// 1.1e-9 at 1e6, here 8.6e-15 and 5.4e-11, by the eigendecomposition 9.7e-15 and
+// 1.4e-10.  It costs 0.1 ms of 1.1 at that size, 2 of 21 at n = 24000.
 //
 // Pivots are taken kPcB at a time: candidates are the largest remaining
 // diagonal entries of kPcB strided groups of indices, their columns of the
@@ -33,10 +45,10 @@
 // host's upper bound, the columns beyond k being zero.
 //
 // B and the shifted B are factorised side by side by the float64 tile Cholesky
-// and B^-2 applied in one launch of its triangular solves (two library
+// and B^-3 applied in one launch of its triangular solves (two library
 // factorisations and eight library solves took 447 us of 1002 at r = 261).
 // Measured at n = 1900, r = 261 (the small configuration): 21.0 ms with the
-// eigendecomposition, 0.9 ms here; n = 24000, r = 1921: 6.9 s and 19 ms.  A
+// eigendecomposition, 1.0 ms here; n = 24000, r = 1921: 6.9 s and 21 ms.  A
 // matrix of full rank is refused after the first steps (by the trace its
 // columns have taken) or at n/2 columns: 0.2 ms lost of 3.3 at n = 300, 0.4 of
 // 28 at n = 2000.
@@ -53,13 +65,18 @@ namespace vtb {
 constexpr int kPcB = 32;               // candidates (and at most as many pivots) per step
 constexpr int kPcMaxRank = 3072;       // columns the workspace holds at most
 constexpr int kPcProbes = 3;            // vectors the remainder is tried on
+constexpr int kPcSweeps = 8;            // refinements at most
+// a refinement of this size (of |c|) leaves its square; one that is still above
+// kPcSettled when they no longer shrink is not rounding (condition numbers reach
+// 1 / rcond <= 1.1e10)
+constexpr double kPcConverged = 1e-8, kPcSettled = 1e-5;
 constexpr double kPcKeep = 0.01;       // accepted pivots, relative to the largest remaining diagonal
 // pivots end here, relative to G's largest diagonal entry: the noise left by
 // the updates is mostly below 1e-13 (1.4e-14 absolute at n = 2000, r = 800), but
 // at n = 24000, r = 1921 one clip in ten had an entry above 1024 eps, took it as
 // a pivot and was refused (6.9 s for 19 ms).  Over 190 matrices of n = 1900 to 24000 the largest entry
 // left was 1960 eps, none was refused.
-// What lies between is judged with the remainder, whose certificate is far
+// What lies between is judged with the remainder, whose test is far
 // stricter than this line.
 constexpr double kPcTol = 4096 * 2.220446049250313e-16;
 
@@ -71,6 +88,7 @@ struct PcState {
     double R[kPcB * kPcB];             // factor of the accepted block, row-major lower
     double trace;                      // of the remainder G - L L^T
     double probe, norm;                // largest |G v - L L^T v|_2 of the probes; |B|_inf
+    double ratio;                      // |last refinement| / |c|
     int info[2];
 };
 
@@ -110,7 +128,7 @@ __global__ void __launch_bounds__(1024) pc_init_kernel(const double* __restrict_
         st->maxd0 = m;
         st->tol = kPcTol * m;
         st->dmax = m;
-        st->probe = st->norm = 0.0;
+        st->probe = st->norm = st->ratio = 0.0;
         st->info[0] = st->info[1] = 0;
     }
 }
@@ -325,9 +343,9 @@ __global__ void __launch_bounds__(1024) pc_gemv_t_kernel(const double* __restric
     }
 }
 
-// y_b = A x_b (+ y_b when add), one warp a row
+// y_b = A x_b, one warp a row
 __global__ void __launch_bounds__(256) pc_gemv_kernel(const double* __restrict__ A, int64_t ld, int n, int r,
-                                                      const double* __restrict__ x, double* __restrict__ y, int add) {
+                                                      const double* __restrict__ x, double* __restrict__ y) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
     const double* xv = x + (int64_t)blockIdx.y * r;
@@ -335,11 +353,16 @@ __global__ void __launch_bounds__(256) pc_gemv_kernel(const double* __restrict__
     for (int j = lane; j < r; j += 32) s = fma(A[(int64_t)i * ld + j], xv[j], s);
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     double* q = y + (int64_t)blockIdx.y * n + i;
-    if (lane == 0) *q = add ? *q + s : s;
+    if (lane == 0) *q = s;
 }
 
 // y_b = G x_b from G's lower triangle, b < NV: the part left of the diagonal
-// by rows (one warp each) into y, then the part below it by columns added
+// by rows (one warp each) into y, then the part below it by columns added.
+// Columns: few blocks at the small configuration (n = 1780), so each takes
+// kPcCols of them and loads kPcRows rows at a time: 13 us (20 for four vectors),
+// against 57 with 32 columns a block and one row at a time.
+constexpr int kPcCols = 16, kPcRows = 8;
+
 template <int NV>
 __global__ void __launch_bounds__(256) pc_symv_rows_kernel(const double* __restrict__ G, int64_t ld, int n,
                                                            const double* __restrict__ x, double* __restrict__ y) {
@@ -362,22 +385,31 @@ __global__ void __launch_bounds__(256) pc_symv_rows_kernel(const double* __restr
 template <int NV>
 __global__ void __launch_bounds__(512) pc_symv_cols_kernel(const double* __restrict__ G, int64_t ld, int n,
                                                            const double* __restrict__ x, double* __restrict__ y) {
-    __shared__ double part[NV][16][33];
-    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, g = threadIdx.x >> 5;
+    constexpr int groups = 512 / kPcCols;
+    __shared__ double part[NV][groups][kPcCols + 1];
+    const int q = threadIdx.x % kPcCols, c = blockIdx.x * kPcCols + q, g = threadIdx.x / kPcCols;
     double s[NV] = {};
     if (c < n)
-        for (int i = blockIdx.x * 32 + g; i < n; i += 16)
-            if (i > c) {
-                const double v = G[(int64_t)i * ld + c];
+        for (int i0 = blockIdx.x * kPcCols + g; i0 < n; i0 += groups * kPcRows) {
+            double v[kPcRows];
 #pragma unroll
-                for (int b = 0; b < NV; ++b) s[b] = fma(v, x[(int64_t)b * n + i], s[b]);
+            for (int k = 0; k < kPcRows; ++k) {
+                const int i = i0 + groups * k;
+                v[k] = i > c && i < n ? G[(int64_t)i * ld + c] : 0.0;
             }
 #pragma unroll
-    for (int b = 0; b < NV; ++b) part[b][g][lane] = s[b];
+            for (int k = 0; k < kPcRows; ++k) {
+                const int i = min(i0 + groups * k, n - 1);
+#pragma unroll
+                for (int b = 0; b < NV; ++b) s[b] = fma(v[k], x[(int64_t)b * n + i], s[b]);
+            }
+        }
+#pragma unroll
+    for (int b = 0; b < NV; ++b) part[b][g][q] = s[b];
     __syncthreads();
     if (g < NV && c < n) {
         double t = 0.0;
-        for (int k = 0; k < 16; ++k) t += part[g][k][lane];
+        for (int k = 0; k < groups; ++k) t += part[g][k][q];
         y[(int64_t)g * n + c] += t;
     }
 }
@@ -402,6 +434,35 @@ __global__ void pc_residual_kernel(const double* __restrict__ q, const double* _
                                    int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) res[i] = q[i] - y[i];
+}
+
+// c += v, st->ratio = |v| / |c| (one block)
+__global__ void __launch_bounds__(1024) pc_correct_kernel(double* __restrict__ c, const double* __restrict__ v, int n,
+                                                          PcState* __restrict__ st) {
+    __shared__ double sm[32], tm[32];
+    double s = 0.0, t = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double u = c[i] + v[i];
+        c[i] = u;
+        s = fma(v[i], v[i], s);
+        t = fma(u, u, t);
+    }
+    for (int o = 16; o; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sm[threadIdx.x >> 5] = s;
+        tm[threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) {
+            s += sm[w];
+            t += tm[w];
+        }
+        st->ratio = s > 0.0 ? sqrt(s / t) : s;       // 0 for q = 0, NaN stays
+    }
 }
 
 // st->probe = the largest |y_b - z_b|_2 (raised to it; one block per probe),
@@ -551,37 +612,51 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
     const Chol64System sys[2] = {{w.B, ldb, r, w.t, w.wk, info, nullptr, 0.0},
                                  {w.B2, ldb, r, w.z, w.wk2, info + 1, nullptr, 0.0}};
     VTB_CUDA_TRY(cudaMemsetAsync(w.z, 0, (size_t)r * 8, s));
-    // c (+)= L B^-1 B^-1 L^T x; the first time with the factorisation, which leaves the first forward solve done
-    auto apply = [&](const double* x, int add) -> int {
+    // y = L B^-3 L^T x; the first time with the factorisation, which leaves the first forward solve done
+    auto apply = [&](const double* x, double* y, bool first) -> int {
         pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, x, w.t);
-        const int f = add ? VTB_OK : chol64_factor(sys, 2, s);
+        const int f = first ? chol64_factor(sys, 2, s) : VTB_OK;
         if (f) return f;
-        const int g = chol64_solve(sys[0], !add, add ? 4 : 3, s);
+        const int g = chol64_solve(sys[0], first, first ? 5 : 6, s);
         if (g) return g;
-        pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, c, add);
+        pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, y);
         return VTB_OK;
     };
-    if ((st = apply(q, 0))) return st;
-    // one pass over G for the refinement (x = c) and the probes
+    const int rows_grid = ceil_div((int64_t)n * 32, 256), cols_grid = ceil_div(n, kPcCols);
+    auto product = [&](const double* x, double* y) {
+        pc_symv_rows_kernel<1><<<rows_grid, 256, 0, s>>>(G, ld, n, x, y);
+        pc_symv_cols_kernel<1><<<cols_grid, 512, 0, s>>>(G, ld, n, x, y);
+    };
+    if ((st = apply(q, w.v, true))) return st;
+    // one pass over G for c and the probes
     constexpr int nv = 1 + kPcProbes;
-    VTB_CUDA_TRY(cudaMemcpyAsync(w.v, c, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
     pc_probes_kernel<<<ceil_div((int64_t)kPcProbes * n, 256), 256, 0, s>>>(w.v + n, n, w.st);
-    pc_symv_rows_kernel<nv><<<ceil_div((int64_t)n * 32, 256), 256, 0, s>>>(G, ld, n, w.v, w.y);
-    pc_symv_cols_kernel<nv><<<ceil_div(n, 32), 512, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_symv_rows_kernel<nv><<<rows_grid, 256, 0, s>>>(G, ld, n, w.v, w.y);
+    pc_symv_cols_kernel<nv><<<cols_grid, 512, 0, s>>>(G, ld, n, w.v, w.y);
     pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), kPcProbes), 1024, 0, s>>>(w.L, w.ldl, n, r, w.v + n, w.t);
-    pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), kPcProbes), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, w.v + n, 0);
+    pc_gemv_kernel<<<dim3(rows_grid, kPcProbes), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, w.v + n);
     pc_probe_kernel<<<kPcProbes, 1024, 0, s>>>(w.y + n, w.v + n, w.d, n, w.st);
-    pc_residual_kernel<<<ceil_div(n, 256), 256, 0, s>>>(q, w.y, w.v, n);
-    if ((st = apply(w.v, 1))) return st;
+    VTB_CUDA_TRY(cudaMemcpyAsync(c, w.y, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
     PcState end;
-    VTB_CUDA_TRY(cudaMemcpyAsync(&end, w.st, sizeof(end), cudaMemcpyDeviceToHost, s));
-    if (kept) VTB_CUDA_TRY(cudaMemcpyAsync(kept, w.st, 4, cudaMemcpyDeviceToDevice, s));
-    VTB_CUDA_TRY(cudaStreamSynchronize(s));
-    st = launch_status();
-    if (st) return st;
+    double last = 1.0;
+    for (int sweep = 0; sweep < kPcSweeps; ++sweep) {
+        product(c, w.v);
+        pc_residual_kernel<<<ceil_div(n, 256), 256, 0, s>>>(q, w.v, w.y, n);
+        product(w.y, w.v);
+        if ((st = apply(w.v, w.y, false))) return st;
+        pc_correct_kernel<<<1, 1024, 0, s>>>(c, w.y, n, w.st);
+        VTB_CUDA_TRY(cudaMemcpyAsync(&end, w.st, sizeof(end), cudaMemcpyDeviceToHost, s));
+        if (sweep == 0 && kept) VTB_CUDA_TRY(cudaMemcpyAsync(kept, w.st, 4, cudaMemcpyDeviceToDevice, s));
+        VTB_CUDA_TRY(cudaStreamSynchronize(s));
+        st = launch_status();
+        if (st) return st;
+        if (end.info[0] != 0 || end.info[1] != 0 || !(end.ratio > kPcConverged) || end.ratio > 0.5 * last) break;
+        last = end.ratio;
+    }
     // the remainder against the rule, with s_0 at least the largest diagonal entry and |B|_inf / sqrt(r)
     const double rule = rcond * std::max(end.maxd0, end.norm / std::sqrt((double)r));
-    if (end.info[0] != 0 || end.info[1] != 0 || !(end.trace <= 0.1 * rule) || !(end.probe <= 0.05 * rule)) return VTB_OK;
+    if (end.info[0] != 0 || end.info[1] != 0 || !(end.ratio <= kPcSettled)) return VTB_OK;
+    if (!(end.trace <= 0.1 * rule) || !(end.probe <= 0.05 * rule)) return VTB_OK;
     *accepted = 1;
     return VTB_OK;
 }
