@@ -66,10 +66,10 @@ __device__ bool rnn_grid_barrier(unsigned* count, unsigned* gen, unsigned nblock
 // eigenvector's part by 1 - dta lambda), so a residual longer than br shows
 // updates that diverge, where the squared maps' rounding grows with the number
 // of updates that each stands for instead of with its square root (402 updates,
-// dta lambda = 2.4 and 3.4: 1.8 times the sum of the updates' own rounding): all updates are then
-// taken here, from 0.  Else x stays.  (kRnnGrowth leaves room for the residual's own
-// rounding.)  Every CTA takes the sums over all rows in the same order and so
-// decides alike.  Measured at K = 1921: 16 us of 2600.
+// dta lambda = 2.4 and 3.4: 1.8 times the sum of the updates' own rounding): all
+// updates are then taken here, from 0.  Else x stays.  (kRnnGrowth leaves room for
+// the residual's own rounding.)  Every CTA takes the sums over all rows in the
+// same order and so decides alike.  Measured at K = 1921: 16 us of 2600.
 constexpr double kRnnGrowth = 1.0 + 1e-6;
 
 template <bool GUARD>
@@ -87,7 +87,9 @@ __global__ void __launch_bounds__(kRnnThreads) rnn_coeff_kernel(const double* __
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     if (GUARD) {
         __shared__ double sums[2][kRnnThreads / 32];
-        if (*(volatile int*)err) return;      // set by the launch before, or by a CTA that gave up: no one is waited for
+        // set by the launch before, or by a CTA that gave up: no one is waited for
+        // (all threads of a CTA by one vote: the word may change while they read it)
+        if (__syncthreads_or(*(volatile int*)err)) return;
         for (int j = threadIdx.x; j < K; j += blockDim.x) sx[j] = __ldcg(x + j);
         __syncthreads();
         for (int r = r0 + warp; r < r1; r += nw) {
