@@ -82,6 +82,37 @@ def test_tiles_of_the_call(K):
     assert int(flags.abs().max()) == 0 and bool(same)
 
 
+@pytest.mark.parametrize("K,extra", [(261, 20), (500, 40)])
+def test_as_close_as_the_library(K, extra):
+    """Against the solution refined in extended precision: as many roundings of
+    the same sizes as a blocked factorisation in float64, so on average the
+    library's error, a quarter left for the samples."""
+    ratios = []
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(100 + seed)
+        B = torch.randn(K, K + extra, dtype=torch.float64, device="cuda", generator=g)
+        M = B @ B.T / K
+        M = 0.5 * (M + M.T)
+        b = M @ torch.randn(K, dtype=torch.float64, device="cuda", generator=g)
+        x, _, flag, _ = _solve(M, b, K + (K & 1))
+        nb = np.zeros(1, np.int64)
+        call("vtb_sym_workspace", K, 1, nb.ctypes.data)
+        work = torch.empty(int(nb[0]), dtype=torch.uint8, device="cuda")
+        A, y = M.clone(), b.clone()
+        st = torch.zeros(4, dtype=torch.float64, device="cuda")
+        call("vtb_sym_factor", dptr(A), K, K, 1, 1e-12, dptr(work), work.numel(), dptr(st), st.data_ptr() + 8, stream_ptr())
+        call("vtb_sym_potrs", dptr(A), K, dptr(y), K, 1, dptr(work), work.numel(), stream_ptr())
+        assert flag == 0
+        Ml, bl = M.cpu().numpy().astype(np.longdouble), b.cpu().numpy().astype(np.longdouble)
+        inv = np.linalg.inv(M.cpu().numpy())
+        exact = y.cpu().numpy().astype(np.longdouble)
+        for _ in range(6):
+            exact = exact + inv @ (bl - Ml @ exact).astype(np.float64)
+        e = [np.sqrt(((v.cpu().numpy() - exact) ** 2).sum()) for v in (x, y)]
+        ratios.append(float(e[0] / e[1]))
+    assert np.exp(np.mean(np.log(ratios))) <= 1.25
+
+
 def test_wait_limit_runs_out_and_recovers():
     M, b = _spd(979, 5)
     with _abi.wait_limit(1):

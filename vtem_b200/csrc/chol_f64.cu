@@ -166,19 +166,28 @@ __device__ __forceinline__ void d_mma(double (&d)[2], double a, double b) {
 
 // rows 8w..8w+7 of acc -= P Q^T (Q[n][k] at k*36 + n) or, TRI, acc += P Q^T with
 // Q lower triangular and k contiguous (Q[n][k] at n*36 + k); columns 8j.. for j < nj.
-// Lane l holds row l / 4, columns 2 (l % 4) + {0, 1} of each 8 x 8 block.
+// Lane l holds row l / 4, columns 2 (l % 4) + {0, 1} of each 8 x 8 block.  The
+// product is summed by itself and then subtracted: taken off the tile one k at a
+// time, every one of K terms is rounded to the tile's own size, and the solve's
+// error was up to twice the library's (windows of K = 221 and 261: 1.1 to 2.3 times
+// it; summed apart 0.3 to 1.0 times, at the same speed).
 template <bool TRI>
 __device__ __forceinline__ void d_product(double (&acc)[4][2], const double* P, const double* Q, int w, int nj) {
     const int lane = threadIdx.x & 31, lo = lane & 3, hi = lane >> 2;
+    double t[4][2] = {};
 #pragma unroll
     for (int kk = 0; kk < kDT; kk += 4) {
         const double p = P[(kk + lo) * kDL + 8 * w + hi];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (TRI ? kk < 8 * j + 8 : j < nj)
-                d_mma(acc[j], TRI ? p : -p, TRI ? Q[(8 * j + hi) * kDL + kk + lo] : Q[(kk + lo) * kDL + 8 * j + hi]);
+                d_mma(t[j], p, TRI ? Q[(8 * j + hi) * kDL + kk + lo] : Q[(kk + lo) * kDL + 8 * j + hi]);
         }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) acc[j][e] = TRI ? acc[j][e] + t[j][e] : acc[j][e] - t[j][e];
 }
 
 __device__ __forceinline__ void d_acc_to(const double (&acc)[4][2], double* s, int w, int nj = 4) {
@@ -258,12 +267,11 @@ __device__ __forceinline__ void d_subst8(double* X, const double* L, const doubl
 __device__ __forceinline__ void d_patch(double* X, const double* L, int r0, int c0, int o) {
     const int lane = threadIdx.x & 31, lo = lane & 3, hi = lane >> 2;
     double* d0 = X + (c0 + 2 * lo) * kDL + r0 + hi;
-    double acc[2] = {d0[0], d0[kDL]};
+    double acc[2] = {0.0, 0.0};
 #pragma unroll
-    for (int kk = 0; kk < 8; kk += 4)
-        d_mma(acc, -X[(o + kk + lo) * kDL + r0 + hi], L[(o + kk + lo) * kDL + c0 + hi]);
-    d0[0] = acc[0];
-    d0[kDL] = acc[1];
+    for (int kk = 0; kk < 8; kk += 4) d_mma(acc, X[(o + kk + lo) * kDL + r0 + hi], L[(o + kk + lo) * kDL + c0 + hi]);
+    d0[0] -= acc[0];
+    d0[kDL] -= acc[1];
 }
 
 __device__ __forceinline__ void d_panel_sync() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
