@@ -451,7 +451,8 @@ int vtb_sym_potrs(const void* Mfac, int64_t ld, double* x, int K, int mode, void
 /* x = M^-1 x in float64 by a Cholesky factorisation in place (lower factor),
  * factor and forward solve in one cooperative launch, the backward solve in a
  * second.  flag and pivots as vtb_sym_factor (3: a bounded wait ran out; M and
- * x are then undefined).  work: vtb_sym_chol_solve_bytes(K) bytes, 256-byte
+ * x are then undefined; -1: solved, but a 32 x 32 diagonal tile of the factor is
+ * so ill conditioned that x may be less exact than by substitution).  work: vtb_sym_chol_solve_bytes(K) bytes, 256-byte
  * aligned. */
 int64_t vtb_sym_chol_solve_bytes(int K);
 int vtb_sym_chol_solve(double* M, int64_t ld, int K, double* x, double rcond, void* work, int64_t work_bytes,

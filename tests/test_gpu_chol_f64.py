@@ -113,6 +113,37 @@ def test_as_close_as_the_library(K, extra):
     assert np.exp(np.mean(np.log(ratios))) <= 1.25
 
 
+def test_ill_conditioned_tiles_are_flagged():
+    """A nearly dependent pair in every eighth row: the inverses of the
+    diagonal tiles then cost digits (Skeel condition numbers of 40 and 10,000)."""
+    for c, want in ((1e1, 0), (1e6, -1)):
+        for K in (300, 31):
+            g = torch.Generator(device="cuda").manual_seed(1)
+            B = torch.randn(K, K + 40, dtype=torch.float64, device="cuda", generator=g)
+            n = B[1::8].shape[0]
+            B[1::8] = B[0::8][:n] + B[1::8] / c ** 0.5
+            assert _solve(B @ B.T / K, B[:, 0].clone(), K + (K & 1), rcond=1e-16)[2] == want
+
+
+def test_short_window_takes_the_library(monkeypatch):
+    """A window of 0.6 temporal periods, the truncation switched off: the
+    coefficients are the library's, bit for bit."""
+    rng = np.random.default_rng(12)
+    N, n, Mx, My, Mt = 60, 3000, 2, 2, 8
+    Ds = rng.standard_normal((N, 2 * My + 1, 2 * Mx + 1)) + 1j * rng.standard_normal((N, 2 * My + 1, 2 * Mx + 1))
+    Ds = 0.5 * (Ds + np.conj(Ds[:, ::-1, ::-1])) * O.ellipse_mask(Mx, My)[None]
+    tk1 = rng.uniform(0, 0.6 * Mt / 20, n)
+    t = [torch.as_tensor(x, device="cuda") for x in (tk1, tk1 + rng.uniform(0.004, 0.03, n),
+                                                     np.sort(rng.integers(0, N, n)).astype(np.int32))]
+    p = [rng.uniform(0.8, 1.2, N), rng.uniform(0.01, 0.05, N), rng.uniform(1, 3, N)]
+    dec = fast.CoeffDecoder(torch.as_tensor(Ds, device="cuda"), rng.uniform(0.5, 1.0, N), Mx, My, 2 * np.pi * 20, Mt,
+                            8, 8, 8, 8, solver="chol", rcond=1e-20)
+    run = lambda: dec.coefficients(*t, *p, assume_sorted=True).clone()
+    a = run()
+    monkeypatch.setattr(fast, "CHOL_TILES_MAX", 0)
+    assert torch.equal(a, run())
+
+
 def test_wait_limit_runs_out_and_recovers():
     M, b = _spd(979, 5)
     with _abi.wait_limit(1):

@@ -617,7 +617,7 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
         pc_gemv_t_kernel<<<dim3(ceil_div(r, 32), 1), 1024, 0, s>>>(w.L, w.ldl, n, r, x, w.t);
         const int f = first ? chol64_factor(sys, 2, s) : VTB_OK;
         if (f) return f;
-        const int g = chol64_solve(sys[0], first, first ? 5 : 6, s);
+        const int g = chol64_solve(sys[0], first, first ? 5 : 6, false, s);
         if (g) return g;
         pc_gemv_kernel<<<dim3(ceil_div((int64_t)n * 32, 256), 1), 256, 0, s>>>(w.L, w.ldl, n, r, w.t, y);
         return VTB_OK;

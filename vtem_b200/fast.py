@@ -418,7 +418,7 @@ class CoeffDecoder(object):
         for i, mode in enumerate(modes):
             if mode == 1:
                 flag, piv = self._chol_tiles(s) if K <= CHOL_TILES_MAX else (3, None)
-                if flag == 3:            # larger, or a wait of the tile solve ran out
+                if flag in (3, -1):      # larger, a wait of the tile solve ran out, or its tiles are ill conditioned
                     flag, piv = self._chol_library(s)
                 self.last_pivots = piv
                 if flag == 0:
@@ -440,7 +440,8 @@ class CoeffDecoder(object):
             return
 
     def _chol_tiles(self, s):
-        """xr = M^-1 br by the tile Cholesky; (flag, pivots), flag 3 when it gave up."""
+        """xr = M^-1 br by the tile Cholesky; (flag, pivots), flag 3 when it gave
+        up, -1 when substitution would be more exact."""
         K = self.K
         if self._chol64 is None:
             self._chol64 = torch.empty(int(lib().vtb_sym_chol_solve_bytes(K)), dtype=torch.uint8, device=self.M.device)
