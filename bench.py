@@ -662,7 +662,9 @@ def measured_traffic(voxels, kernel):
 
 def run_plain(w, prep, tk1, tk2, ind, u_fast_variants, dev, Nt):
     """The plain float64 path of the reference on the whole clip: analytic
-    n x n Gram, eigendecomposition pseudoinverse, synthesis."""
+    n x n Gram, pseudoinverse (the low-rank solve, or the eigendecomposition where
+    it does not apply; stage "pinv_eigh"), synthesis.  One cold pass: gigabytes
+    are allocated inside the timed stages and released before the synthesis."""
     import torch
     from vtem_b200 import dirichlet, linalg
 

@@ -232,7 +232,8 @@ int vtb_solve_eq_sym(double* G, int64_t ld, const double* q, double* c, int n, d
  * to be such a matrix (for an indefinite G by pseudo-random probes of
  * G - L L^T); else 0, and the caller solves with vtb_solve_eq_sym: G (its lower
  * triangle is read) is not written either way.  *kept (device, may be NULL)
- * receives r.  Synchronises the stream. */
+ * receives r.  Synchronises the stream.  The workspace holds the factor,
+ * n x min(n/2, 3072) doubles, and a few square matrices of that order. */
 int vtb_solve_psd_workspace(int n, int64_t* bytes);
 int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* c, int n, double rcond, void* work,
                   int64_t work_bytes, int32_t* kept, int32_t* accepted, void* stream);
@@ -285,7 +286,8 @@ int vtb_coeff_temporal_gram(const double* tk1, const double* tk2, const int32_t*
                             double W, double* Wn, double* gn, void* stream);
 
 /* M = sum_n (d_n d_n^H) kron Wn (column-major, K x K complex, ld ldm) and
- * b = sum_n d_n kron gn. */
+ * b = sum_n d_n kron gn.  Every Wn is Hermitian, as vtb_coeff_temporal_gram
+ * gives it: only its entries m <= m' are read. */
 int vtb_coeff_gram(const double* d, int N, int Ks, const double* Wn, const double* gn, int Kt, double* M,
                    int64_t ldm, double* b, void* stream);
 
@@ -559,7 +561,9 @@ int vtb_sym_pinv(double* M, int64_t ld, const double* b, double* x, int K, doubl
  * inverses of each factor's 32 x 32 diagonal blocks for vtb_sym_potrs_batched
  * (Dinv + z * vtb_sym_dinv_floats(K)).  infos (device) receives cuSOLVER's
  * per-system status.  The grouped counterpart of the per-window solve of
- * vtem/vtdm.py:645-648.  Does not synchronise. */
+ * vtem/vtdm.py:645-648.  Does not synchronise.  Superseded, with
+ * vtb_sym_potrs_batched, by vtb_chol_batch_factor and vtb_chol_batch_solve,
+ * which the batch decoder uses. */
 int vtb_sym_factor_batched(float** Mptrs, int64_t ld, int K, int batch, double rcond, float* Dinv, int32_t* infos,
                            int32_t* flags, double* pivots, void* stream);
 int64_t vtb_sym_dinv_floats(int K);
@@ -591,7 +595,7 @@ int vtb_sym_pinv_batched(double* M, const double* b, double* x, int K, int batch
  * spike Gram (vtem/neural_network.py:15-128) mapped by a = Phi^H c
  * (Phi^H c_{i+1} = Phi^H c_i + dt_alpha (Phi^H q - Phi^H Phi Phi^H c_i)), on
  * K x K instead of n x n.  One cooperative launch runs every update (rows of
- * Mr cached in shared memory); x_tmp (K doubles) and bar (16 bytes) are
+ * Mr cached in shared memory); the decoder uses vtb_rnn_coeff_work.  x_tmp (K doubles) and bar (16 bytes) are
  * scratch.  After the stream reaches the call's end, the int32 at byte
  * offset 8 of bar is nonzero if a grid-barrier wait exceeded its limit (the
  * result is then invalid). */
@@ -601,7 +605,9 @@ int vtb_rnn_coeff(const double* Mr, int64_t ld, const double* br, double* x, dou
 /* The same iterate as vtb_rnn_coeff for symmetric Mr, by repeated squaring of
  * the update's map (a few float64 products in place of most of the exchanges
  * between SMs), all scratch in one workspace (256-byte aligned),
- * which begins with vtb_rnn_coeff's status words.  The form the decoder uses. */
+ * which begins with vtb_rnn_coeff's status words.  Updates that diverge
+ * (dt_alpha above 2 / lambda_max) are taken one by one instead, bit for bit
+ * vtb_rnn_coeff's.  The form the decoder uses. */
 int vtb_rnn_coeff_workspace(int K, int64_t* bytes);
 int vtb_rnn_coeff_work(const double* Mr, int64_t ld, const double* br, double* x, int K, double dt_alpha, int steps,
                        void* work, int64_t work_bytes, void* stream);

@@ -595,7 +595,9 @@ VTB_API int vtb_dirichlet_coeffs(const double* rf, int N, int LPy, int LPx, int6
     const int Kx = 2 * Mx + 1, Ky = 2 * My + 1;
     VTB_CHECK_ARG(Kx * Ky <= 256);
     // the tensor path needs its tables and one RF's row sums in shared memory
-    // (256 x 256: 74 KB, three blocks per SM); longer sides and more bins take the general kernel
+    // (256 x 256: 74 KB beside 16 KB of partial sums, two blocks per SM); longer
+    // sides and more bins take the general kernel.  Where fewer blocks fit on an
+    // SM than the grid counts on (sides of 144 to 200), the others follow.
     const int Xp = (LPx + 7) & ~7, Yp = (LPy + 15) & ~15;
     const size_t smm = (size_t)(2 * Yp + (LPx == LPy && Mx == My ? 0 : Xp)) * kDfS * sizeof(double);
     if (Kx <= 16 && Ky <= 16 && smm <= kCallSmem) {

@@ -195,8 +195,8 @@ class Server(object):
     # -- phase 2: batched Cholesky (loop thread, solve stream) --------------
     def _launch_chol(self, jobs):
         """Launch the grouped mixed-precision solve of ``jobs`` (all with a
-        coefficient-space system staged by the encoder): one batched float32
-        Cholesky per system size, batched triangular solves, float64
+        coefficient-space system staged by the encoder): one launch that factorises
+        and inverts every system in float32, batched product solves, float64
         refinement sweeps; returns a handle whose ``query()`` tells when it
         is done and ``flags()`` then lists, per job, whether the float64 path
         must solve it instead."""
