@@ -110,16 +110,13 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p
     const int k_lo = SPLIT ? (int)((int64_t)slabs * blockIdx.z / splits) : 0;
     const int nk = SPLIT ? (int)((int64_t)slabs * (blockIdx.z + 1) / splits) : slabs;
     const int fr = lane >> 2, fk = lane & 3;
-    double acc[MT][NT][4];   // (C = A^2 + beta A: the addend first, so that the sum is one chain of FMAs)
+    double acc[MT][NT][4];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const int gm = m0 + wm + 16 * i + 8 * (h >> 1) + fr, gn = n0 + wn + 8 * j + 2 * fk + (h & 1);
-                acc[i][j][h] = MODE == kSym && gm < p.M && gn < p.N ? p.beta * p.A[(int64_t)gm * p.a_m + gn] : 0.0;
-            }
+            for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
     SA la;
     SB lb;
     la.init(p.A, p.a_m, p.a_k, m0, k_lo * kBK, p.M);
@@ -173,7 +170,8 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_f64_kernel(GemmF64Args p
                     const int gm = m0 + wm + 16 * i + 8 * (h >> 1) + fr, gn = n0 + wn + 8 * j + 2 * fk + (h & 1);
                     if constexpr (MODE == kSym) {
                         if (gm >= p.M || gn >= p.N) continue;
-                        const double v = acc[i][j][h];
+                        // the addend last: with it first, every one of N terms is rounded to its size
+                        const double v = fma(p.beta, p.A[(int64_t)gm * p.a_m + gn], acc[i][j][h]);
                         p.C[(int64_t)gm * p.c_m + gn] = v;
                         if (m0 != n0) p.C[(int64_t)gn * p.c_m + gm] = v;
                     } else {
