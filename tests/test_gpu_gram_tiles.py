@@ -39,3 +39,32 @@ def test_gram_tiles_match_oracle(n, Mt, lower, lamb, shift):
     assert np.abs(G - Go)[keep].max() <= tol
     assert np.abs(G1 - Go)[keep].max() <= tol
     assert np.all(G1[~keep] == 7.0)
+
+
+@pytest.mark.parametrize("T,Mt,shift", [(0.3, 4, 0.0), (1.0, 8, 0.0), (3.0, 8, 100.0), (2.0, 12, 0.0)])
+@pytest.mark.parametrize("table", [True, False])
+def test_error_does_not_grow_with_time(T, Mt, shift, table):
+    """Against the entries in extended precision: the interval's harmonics are
+    powers and products of at most eight correctly rounded factors (two units of
+    rounding each on average, squared entries: four in all), whatever phase m W t
+    they stand for.  Cosines of rounded arguments are off by m W t units."""
+    rng = np.random.default_rng(Mt)
+    n, Wt, L = 300, 2 * np.pi * 20, np.longdouble
+    a = rng.uniform(0, T, n) + shift
+    b = a + rng.uniform(0.02, 0.06, n)
+    W, one = Wt / Mt, np.ones(1)
+    al, bl = a.astype(L) - L(a[0]), b.astype(L) - L(a[0])
+    rows = [bl - al]
+    for m in range(1, Mt + 1):
+        k = m * L(W)
+        rows += [np.sqrt(L(2)) * (np.sin(k * bl) - np.sin(k * al)) / k, np.sqrt(L(2)) * (np.cos(k * al) - np.cos(k * bl)) / k]
+    R = np.stack(rows, 1)
+    want = R @ R.T
+    cp = dirichlet.dirichlet(1, a, b, np.zeros(n, np.int32), one, one, one, one, Wt, Mt)
+    cp.compute_G(np.ones((1, 1)))
+    if not table:
+        Dd = dirichlet._dev(np.ones((1, 1)))
+        call("vtb_compute_G", dptr(cp.d_tk1), dptr(cp.d_tk2), dptr(cp.d_neuron_ind), n, Wt, Mt, dptr(Dd), 1, 0.0, 0,
+             dptr(cp.d_G), n, stream_ptr())
+    G = cp.d_G.cpu().numpy()
+    assert np.sqrt(((G - want) ** 2).sum() / (want ** 2).sum()) <= 4 * np.finfo(np.float64).eps

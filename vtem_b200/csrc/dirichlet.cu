@@ -359,8 +359,7 @@ __global__ void compute_q_kernel(const double* __restrict__ tk1, const double* _
 //   T_k(m) = int_{tk1}^{tk2} e^{jmWs} ds = (2/(mW)) sin(mW d/2) e^{jmW tbar},
 // so an entry costs 2Mt+1 float64 FMAs instead of 4 Mt cosines, and no
 // difference of cosines cancels.  Only differences of times count: they are
-// taken from the first interval's start, so that an offset common to all
-// costs no phase.  Bound: the HBM write of G (n^2 * 8 bytes).
+// taken from the first interval's start.  Bound: the HBM write of G (n^2 * 8 bytes).
 //
 // A block forms 64 x 64 tiles of the lower triangle of tiles on the float64
 // tensor-core path (mma m8n8k4, exact float64 FMAs: few shared-memory reads
@@ -394,24 +393,56 @@ __device__ __forceinline__ int g_at(int r, int c) { return r * kGT + (c ^ (((r &
 // 2q, 2q + 1 hold the tile's q, q + 4, so that a fragment's stores are contiguous
 __device__ __forceinline__ int g_col(int c) { return (c & ~7) | ((c & 3) << 1) | ((c >> 2) & 1); }
 
-// Harmonics m0 .. m0+kGHarm-1 (m >= 1; zero beyond Mt) of the interval (a, b),
-// scaled: f[S * (2i + 1)] = Re, f[S * (2i + 2)] = Im, and f[0] = b - a in the first pass.
+// a number as a double and its rounding error (error-free sums and products:
+// Knuth's two-sum, one FMA)
+struct GPair {
+    double hi, lo;
+};
+
+__device__ __forceinline__ GPair g_sum(double a, double b) {
+    const double s = a + b, t = s - a;
+    return GPair{s, (a - (s - t)) + (b - t)};
+}
+
+// k x to twice the precision, and its sine and cosine
+__device__ __forceinline__ GPair g_times(double k, const GPair& x) {
+    const double p = __dmul_rn(k, x.hi);
+    return GPair{p, fma(k, x.hi, -p) + k * x.lo};
+}
+
+__device__ __forceinline__ void g_sincos(const GPair& x, double* s, double* c) {
+    double s0, c0;
+    sincos(x.hi, &s0, &c0);
+    *s = fma(c0, x.lo, s0);
+    *c = fma(-s0, x.lo, c0);
+}
+
+// Harmonics m0 .. m0+kGHarm-1 (m >= 1; zero beyond Mt) of the interval (t1, t2)
+// from the origin t0, scaled: f[S * (2i + 1)] = Re, f[S * (2i + 2)] = Im, and
+// f[0] = t2 - t1 in the first pass.  The phases are formed to twice the
+// precision: all harmonics of an interval share them, so that a rounded phase
+// moves the whole interval.  Relative error of G over a window of 1 s, Mt = 8:
+// 1.2e-15 by a cosine per difference of times, 2.1e-15 by rounded phases, 3e-16
+// here.
 template <int S>
-__device__ __forceinline__ void g_features(double a, double b, int m0, int Mt, double W, double scale,
+__device__ __forceinline__ void g_features(double t1, double t2, double t0, int m0, int Mt, double W, double scale,
                                            double* __restrict__ f) {
-    const double d = b - a, tb = 0.5 * (a + b);
-    f[0] = m0 == 1 ? d : 0.0;
+    const GPair a = g_sum(t1, -t0), b = g_sum(t2, -t0), d = g_sum(t2, -t1);
+    GPair tb = g_sum(a.hi, b.hi);
+    tb.lo += a.lo + b.lo;
+    const GPair ph = g_times(0.5 * W, tb), pd = g_times(0.5 * W, d);
+    f[0] = m0 == 1 ? d.hi : 0.0;
     double s1, c1, sh, ch, sp, cp, sq, cq;
-    sincos(W * tb, &s1, &c1);
-    sincos(0.5 * W * d, &sh, &ch);
+    g_sincos(ph, &s1, &c1);
+    g_sincos(pd, &sh, &ch);
     if (m0 == 1) {
         sp = s1;
         cp = c1;
         sq = sh;
         cq = ch;
     } else {
-        sincos(m0 * W * tb, &sp, &cp);
-        sincos(m0 * (0.5 * W) * d, &sq, &cq);
+        g_sincos(g_times(m0, ph), &sp, &cp);
+        g_sincos(g_times(m0, pd), &sq, &cq);
     }
 #pragma unroll
     for (int i = 0; i < kGHarm; ++i) {
@@ -435,9 +466,8 @@ __global__ void __launch_bounds__(128) harmonics_table_kernel(const double* __re
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int m0 = 1 + blockIdx.y * kGHarm;
     if (i >= n) return;
-    const double t0 = tk1[0];
     double f[kGF];
-    g_features<1>(tk1[i] - t0, tk2[i] - t0, m0, Mt, W, 1.0, f);
+    g_features<1>(tk1[i], tk2[i], tk1[0], m0, Mt, W, 1.0, f);
     if (m0 == 1) table[i] = f[0];
 #pragma unroll
     for (int h = 0; h < kGHarm; ++h) {
@@ -543,11 +573,10 @@ __global__ void __launch_bounds__(256, 4) compute_G_kernel(const double* __restr
                 if (rows) g_load<false>(table, n, row0, m0, nf, 1.0, fr);
             } else if (tid < kGT) {
                 const int c = col0 + tid;
-                g_features<kGS>(c < n ? tk1[c] - t0 : 0.0, c < n ? tk2[c] - t0 : 0.0, m0, Mt, W, 2.0,
-                                fc + g_col(tid));
+                g_features<kGS>(c < n ? tk1[c] : t0, c < n ? tk2[c] : t0, t0, m0, Mt, W, 2.0, fc + g_col(tid));
             } else if (tid < 2 * kGT && rows) {
                 const int r = row0 + tid - kGT;
-                g_features<kGS>(r < n ? tk1[r] - t0 : 0.0, r < n ? tk2[r] - t0 : 0.0, m0, Mt, W, 1.0, fr + tid - kGT);
+                g_features<kGS>(r < n ? tk1[r] : t0, r < n ? tk2[r] : t0, t0, m0, Mt, W, 1.0, fr + tid - kGT);
             }
             if (m0 == 1 && tid >= 192) ci[tid - 192] = col0 + tid - 192 < n ? ind[col0 + tid - 192] : 0;
             __syncthreads();
