@@ -163,3 +163,24 @@ def test_synth_rank_long_frame_ranges(Nt):
     assert torch.isfinite(u).all()
     err = float((u - ref).abs().max() / ref.abs().max())
     assert err <= 1e-12, err
+
+
+@pytest.mark.parametrize("t0", [0.0, 3.0, -20.7])
+@pytest.mark.parametrize("Mt", [2, 8, 10])
+def test_synthesis_error_does_not_grow_with_time(t0, Mt):
+    """Against the harmonics in extended precision: the centre angle of a block of
+    frames is formed to twice the precision, so what is rounded are the powers of
+    two unit numbers (at most ten products each) and 2Mt+1 terms."""
+    from vtem_b200._abi import call, stream_ptr
+    rng = np.random.default_rng(Mt)
+    P, Nt, dt, L = 70, 1500, 1e-4, np.longdouble
+    W, Kt = 2 * np.pi * 20 / Mt, 2 * Mt + 1
+    H = rng.standard_normal((P, Kt))
+    Hd = torch.as_tensor(H, device="cuda")
+    u = torch.empty((Nt, P), dtype=torch.float64, device="cuda")
+    call("vtb_synth_harmonics", Hd.data_ptr(), Kt, P, Mt, W, t0, dt, Nt, u.data_ptr(), 0, stream_ptr())
+    th = L(W) * (L(t0) + np.arange(Nt).astype(L) * L(dt))
+    C = np.stack([np.ones(Nt, L)] + [f(m * th) for m in range(1, Mt + 1) for f in (np.cos, np.sin)], 1)
+    want = C @ H.T.astype(L)
+    rel = np.sqrt(((u.cpu().numpy() - want) ** 2).sum() / (want ** 2).sum())
+    assert rel <= (8 + Mt) * np.finfo(np.float64).eps
