@@ -31,7 +31,7 @@
 // against the known solution, for the spectra 1..1/cond of n = 1900, r = 261 and a q
 // outside the range: by L B^-2 L^T refined with q - G c 1.3e-13 at cond = 1e2 and
 // 1.1e-9 at 1e6, here 8.6e-15 and 5.4e-11, by the eigendecomposition 9.7e-15 and
-// 1.4e-10.  It costs 0.1 ms of 1.1 at that size, 2 of 21 at n = 24000.
+// 1.4e-10.  It costs 0.1 ms of 1.0 at that size, 2 of 21 at n = 24000.
 //
 // Pivots are taken kPcB at a time: candidates are the largest remaining
 // diagonal entries of kPcB strided groups of indices, their columns of the
@@ -48,10 +48,11 @@
 // and B^-3 applied in one launch of its triangular solves (two library
 // factorisations and eight library solves took 447 us of 1002 at r = 261).
 // Measured at n = 1900, r = 261 (the small configuration): 21.0 ms with the
-// eigendecomposition, 1.0 ms here; n = 24000, r = 1921: 6.9 s and 21 ms.  A
-// matrix of full rank is refused after the first steps (by the trace its
-// columns have taken) or at n/2 columns: 0.2 ms lost of 3.3 at n = 300, 0.4 of
-// 28 at n = 2000.
+// eigendecomposition, 1.0 ms here; n = 24000, r = 1921: 6.9 s and 21 ms.  What a
+// refusal costs: a matrix of full rank whose spectrum is flat, or an indefinite
+// one, goes after the second step (by the trace its columns have taken), 0.1 ms
+// of 3.3 at n = 300 and of 28 at n = 2000; one whose eigenvalues decay over five
+// decades only at n/2 columns, 0.4 of 3.3 and 2.0 of 27.5.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -593,7 +594,7 @@ VTB_API int vtb_solve_psd(const double* G, int64_t ld, const double* q, double* 
         }
         pc_factor_kernel<<<1, 32, 0, s>>>(w.C, w.st);
         pc_update_kernel<<<ceil_div(n, 64), 64, 0, s>>>(w.C, n, w.L, w.ldl, w.d, w.st);
-        if (step % kCheck == kCheck - 1 || step + 1 == most) {
+        if (step % kCheck == 1 || step + 1 == most) {   // the first look as soon as the trace can refuse
             VTB_CUDA_TRY(cudaMemcpyAsync(&host, w.st, sizeof(host), cudaMemcpyDeviceToHost, s));
             VTB_CUDA_TRY(cudaStreamSynchronize(s));
         }

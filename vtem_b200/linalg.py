@@ -9,8 +9,9 @@ from ._abi import call, dptr, stream_ptr
 
 F64 = torch.float64
 
-# below this size the low-rank solve's steps (0.7 ms at n = 500, against 5.0 for
-# the eigendecomposition) save little and a refusal costs most
+# below this size the low-rank solve's steps (0.7 ms at n = 500, against 5.5 for
+# the eigendecomposition) save little and a refusal costs most (at n = 300 0.1 to
+# 0.4 ms of 3.3)
 PSD_MIN_SIZE = 256
 
 
